@@ -1,0 +1,502 @@
+// DG and Helmholtz operators: set-up (geometry, penalties, neighbours), kernel
+// dispatch and the batched launch.  A template on the number type, instantiated
+// by operator_dg_f64.cu and operator_dg_f32.cu.
+#pragma once
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+
+#include "autotune.hpp"
+#include "kernels_dg.cuh"
+#include "kernels_dg2.cuh"
+#include "kernels_dg3.cuh"
+#include "op_shapes.hpp"
+#include "operator.hpp"
+#include "operator_parts.hpp"
+
+namespace sfem {
+
+namespace {
+
+// ------------------------------------------------------------------ DG ----
+template <typename T>
+class DGOperator final : public Operator {
+ public:
+  DevBuf<T> d_geo;      // [6 + 4 + (mass?1:0)][n_cells]
+  DevBuf<int32_t> d_nb; // [4][n_cells]
+  DevBuf<int8_t> d_nbf; // [4][n_cells]
+  DevBuf<T> d_Q;        // published face normal derivatives: [n_cells][4][NC][NFQ], or block-major
+                        // (scalar problems, 1-thread-per-cell forms), for whole 128-cell blocks
+  DevBuf<int> d_status; // timeouts of the bounded waits in the bulk-copy trace pass
+  bool has_mass = false;
+
+  DGOperator(const Mesh& mesh, const OpConfig& c) {
+    cfg = c;
+    const int p = cfg.degree;
+    K = k_of(p);
+    n_cells = mesh.n_cells;
+    m = int64_t(K) * cfg.n_components * n_cells;
+    n_interior_faces = mesh.n_interior_faces;
+    n_boundary_faces = mesh.n_boundary_faces;
+    has_mass = cfg.kind == FEM_HELMHOLTZ;
+    constrained.assign(m, 0);
+    support.resize(3 * size_t(K) * n_cells);
+    for (int64_t cc = 0; cc < n_cells; ++cc) {
+      const int32_t* cv = &mesh.cell_vertices[4 * cc];
+      for (int i = 0; i < K; ++i)
+        for (int a = 0; a < 3; ++a) {
+          double sum = 0;
+          for (int v = 0; v < 4; ++v) {
+            const int lat = p == 1 ? ref::Tables<1>::LATTICE[i][v]
+                                   : p == 2 ? ref::Tables<2>::LATTICE[i][v] : ref::Tables<3>::LATTICE[i][v];
+            sum += lat * mesh.x[3 * size_t(cv[v]) + a];
+          }
+          support[3 * (size_t(K) * cc + i) + a] = sum / p;
+        }
+    }
+    const int n_geo = has_mass ? 11 : 10;
+    std::vector<T> geo(size_t(n_geo) * n_cells);
+    // per-cell quantities for the penalty
+    std::vector<double> tau(n_cells), inv_h(4 * size_t(n_cells)), area(4 * size_t(n_cells));
+    std::vector<double> absdet(n_cells);
+    for (int64_t cc = 0; cc < n_cells; ++cc) {
+      const CellGeometry g = cell_geometry(mesh, cc);
+      absdet[cc] = std::fabs(g.det);
+      double G[6];
+      metric(g, G);
+      for (int k = 0; k < 6; ++k) geo[size_t(k) * n_cells + cc] = T(G[k]);
+      if (has_mass) geo[size_t(10) * n_cells + cc] = T(cfg.mass * absdet[cc]);
+      double surf = 0;
+      for (int f = 0; f < 4; ++f) {
+        double a, nrm[3];
+        face_area_normal(mesh, cc, f, a, nrm);
+        area[4 * cc + f] = a;
+        inv_h[4 * cc + f] = 2.0 * a / absdet[cc];  // |grad lambda_f| = 1/h_f
+        surf += a * (mesh.nb[4 * cc + f] == -1 ? 1.0 : 0.5);  // -2: interior, neighbour not local
+      }
+      tau[cc] = surf / (absdet[cc] / 6.0);
+    }
+    const double factor = cfg.penalty == FEM_PENALTY_SQUARE ? double((p + 1) * (p + 1))
+                                                            : double((p + 1) * (p + 3)) / 3.0;
+    for (int64_t cc = 0; cc < n_cells; ++cc)
+      for (int f = 0; f < 4; ++f) {
+        const int32_t nbc = mesh.nb[4 * cc + f];
+        double sigma;
+        if (cfg.kind == FEM_HELMHOLTZ) {
+          // 1/h normal to the face, averaged over both sides
+          // (application_helmholtz.cc:1329-1333 and :857-859 on the boundary)
+          sigma = nbc >= 0 ? factor * 0.5 * (inv_h[4 * cc + f] + inv_h[4 * size_t(nbc) + mesh.nbf[4 * cc + f]])
+                           : factor * inv_h[4 * cc + f];
+        } else {
+          // max of the two cells' surface/volume (DG/cells_batched/application.cc:1377-1379)
+          sigma = nbc >= 0 ? factor * std::max(tau[cc], tau[nbc]) : factor * tau[cc];
+        }
+        geo[size_t(6 + f) * n_cells + cc] = T(sigma * area[4 * cc + f]);
+      }
+    d_geo.upload(geo);
+    std::vector<int32_t> nb(4 * size_t(n_cells));
+    std::vector<int8_t> nbf(4 * size_t(n_cells));
+    for (int64_t cc = 0; cc < n_cells; ++cc)
+      for (int f = 0; f < 4; ++f) {
+        nb[size_t(f) * n_cells + cc] = std::max(mesh.nb[4 * cc + f], -1);
+        nbf[size_t(f) * n_cells + cc] = mesh.nbf[4 * cc + f] < 0 ? 0 : mesh.nbf[4 * cc + f];
+      }
+    d_nb.upload(nb);
+    d_nbf.upload(nbf);
+    d_Q.alloc(size_t((n_cells + kQB - 1) / kQB * kQB) * 4 * cfg.n_components * nfq_of(p));
+    d_status.alloc(1);
+    SFEM_CUDA(cudaMemset(d_status.p, 0, sizeof(int)));
+  }
+
+  int status(bool clear) override {
+    int v = 0;
+    SFEM_CUDA(cudaMemcpy(&v, d_status.p, sizeof(int), cudaMemcpyDeviceToHost));
+    if (clear && v) SFEM_CUDA(cudaMemset(d_status.p, 0, sizeof(int)));
+    return v;
+  }
+
+  DGProblem<T> problem(const void* src, void* dst) const {
+    DGProblem<T> pr;
+    pr.geo = d_geo.p;
+    pr.nb = d_nb.p;
+    pr.nbf = d_nbf.p;
+    pr.src = static_cast<const T*>(src);
+    pr.dst = static_cast<T*>(dst);
+    pr.Q = d_Q.p;
+    pr.n_cells = n_cells;
+    return pr;
+  }
+
+  void vmult(void* dst, const void* src, cudaStream_t s) override {
+    const DGProblem<T> pr = problem(src, dst);
+    launch_dg(cfg, &pr, 1, s, 0, d_status.p);
+  }
+
+  void vmult_phase(void* dst, const void* src, int phase, cudaStream_t s) override {
+    const DGProblem<T> pr = problem(src, dst);
+    launch_dg(cfg, &pr, 1, s, phase, d_status.p);
+  }
+
+  size_t scratch_bytes() const override { return d_Q.n * sizeof(T); }
+
+  void vmult_with_scratch(void* dst, const void* src, void* scratch, size_t bytes, cudaStream_t s) override {
+    SFEM_REQUIRE(bytes >= scratch_bytes(), FEM_ERR_ARG, "vmult: scratch too small");
+    DGProblem<T> pr = problem(src, dst);
+    pr.Q = static_cast<T*>(scratch);
+    launch_dg(cfg, &pr, 1, s, 0, d_status.p);
+  }
+
+  void diagonal(void* diag, cudaStream_t s) override {
+    const DGProblem<T> pr = problem(nullptr, diag);
+    launch_dg(cfg, &pr, 1, s, 3, d_status.p);
+  }
+
+  void work(double& flops, double& bytes) const override {
+    const int p = cfg.degree, kq = kq_of(p), nf = nf_of(p), nfq = nfq_of(p), nz = nnz_grad_rt(p);
+    const double trace = 2.0 * (nz + 12 * nfq);
+    double apply = 2.0 * (2 * nz + 9 * kq + 3 * kq * kq) +
+                   4 * 2.0 * (3 * nfq + nf + nf * nf + nf + 2 * nf * nfq + 3 * nfq + 3 * nfq);
+    if (has_mass) apply += 2.0 * (K * K + K);
+    flops = (trace + apply) * cfg.n_components * double(n_cells);
+    const double s = double(sizeof(T));
+    bytes = 2 * s * double(m) + 6 * s * double(n_cells) + double(n_interior_faces) * (8 + s) +
+            double(n_boundary_faces) * (4 + s);
+  }
+
+  // Dispatch over n problems.  what: 0 trace+apply, 1 trace, 2 apply, 3 diagonal.
+  // status: device word set by the bounded waits of the bulk-copy trace pass.
+  static void launch_dg(const OpConfig& cfg, const DGProblem<T>* probs, int n, cudaStream_t s, int what,
+                        int* status) {
+    const bool mass = cfg.kind == FEM_HELMHOLTZ;
+    const int nc = cfg.n_components;
+    SFEM_REQUIRE(nc == 1 || nc == 3, FEM_ERR_ARG, "DG: n_components must be 1 or 3");
+    SFEM_REQUIRE(n >= 1 && n <= kMaxBatch, FEM_ERR_ARG, "DG: 1..40 problems per launch");
+    const int variant = cfg.kernel_variant > 0 ? cfg.kernel_variant : default_variant(cfg.degree, nc);
+#define SFEM_DG_CASE(P, NC, MASS)                                                       \
+  if (cfg.degree == P && nc == NC && mass == MASS) {                                    \
+    run<P, NC, MASS>(probs, n, s, what, variant, status);                               \
+    return;                                                                             \
+  }
+    SFEM_DG_CASE(1, 1, false) SFEM_DG_CASE(2, 1, false) SFEM_DG_CASE(3, 1, false)
+    SFEM_DG_CASE(1, 1, true) SFEM_DG_CASE(2, 1, true) SFEM_DG_CASE(3, 1, true)
+    SFEM_DG_CASE(1, 3, true) SFEM_DG_CASE(2, 3, true) SFEM_DG_CASE(3, 3, true)
+    SFEM_DG_CASE(1, 3, false) SFEM_DG_CASE(2, 3, false) SFEM_DG_CASE(3, 3, false)
+#undef SFEM_DG_CASE
+    throw Error(FEM_ERR_ARG, "DG: unsupported degree/components combination");
+  }
+
+  // kernel forms: 1 thread per cell, 128 cells per CTA; 2 thread per cell, 64
+  // cells per CTA; 3 warp roles, 32 cells per CTA
+  // (measured on B200: scalar P3 runs best register-capped at 64 cells per CTA,
+  // the 3-component forms at 128 cells per CTA)
+  // measured on B200 (DG P3 32^3, medians of 25 L2-flushed vmults): FP64
+  // 82.9 us with 128 cells per CTA against 85.0 us with 64; FP32 44.1 us with
+  // the results in registers and 8 CTAs per SM against 52.2 us; 128 cells per
+  // CTA otherwise
+  static int default_variant(int p, int nc) { return (nc == 1 && p == 3 && sizeof(T) == 4) ? 4 : 1; }
+
+  static DGBatch<T> make_batch(const DGProblem<T>* probs, int n, int bs, int64_t& n_blocks) {
+    DGBatch<T> b;
+    b.n = n;
+    b.block_begin[0] = 0;
+    for (int i = 0; i < n; ++i) {
+      b.p[i] = probs[i];
+      b.block_begin[i + 1] = b.block_begin[i] + (probs[i].n_cells + bs - 1) / bs;
+    }
+    n_blocks = b.block_begin[n];
+    return b;
+  }
+
+  template <class K>
+  static void opt_in_smem(K kernel, size_t bytes, std::atomic<uint64_t>& configured) {
+    int dev = 0;
+    SFEM_CUDA(cudaGetDevice(&dev));
+    once_per_device(configured, dev, [&] {
+      SFEM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+    });
+  }
+
+  // The bulk-copy trace pass needs every copy 16-byte aligned and a whole
+  // number of 16-byte units: src rows (the last block's included) and the
+  // metric rows of the geometry.
+  template <int P>
+  static bool trace_tma_ok(const DGProblem<T>* probs, int n) {
+    for (int i = 0; i < n; ++i) {
+      const DGProblem<T>& pr = probs[i];
+      if ((reinterpret_cast<uintptr_t>(pr.src) | reinterpret_cast<uintptr_t>(pr.geo)) & 15u) return false;
+      if ((size_t(pr.n_cells) * sizeof(T)) % 16 != 0) return false;  // metric row starts
+      if ((size_t(pr.n_cells % kQB) * k_of(P) * sizeof(T)) % 16 != 0) return false;
+    }
+    return true;
+  }
+  template <int P>
+  static void run_trace_tma(const DGBatch<T>& b, int64_t n_blocks, cudaStream_t s, int* status) {
+    constexpr int NS = 3;
+    using S = TraceTmaShape<T, gen::Ops<P>::K, NS>;
+    auto kern = dg_trace_tma_kernel<P, T, NS>;
+    static std::atomic<uint64_t> conf{0};
+    static int grid_per_dev[64] = {};
+    int dev = 0;
+    SFEM_CUDA(cudaGetDevice(&dev));
+    once_per_device(conf, dev, [&] {
+      SFEM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM));
+      int sms = 0, occ = 0;
+      SFEM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+      SFEM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kQB, S::SMEM));
+      SFEM_REQUIRE(occ > 0, FEM_ERR_CUDA, "DG trace pass does not fit on an SM");
+      grid_per_dev[dev] = sms * occ;
+    });
+    const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(n_blocks, grid_per_dev[dev]));
+    kern<<<unsigned(grid), kQB, S::SMEM, s>>>(b, n_blocks, status);
+  }
+
+  // PDLM > 0 (scalar problems): the apply pass is launched as a programmatic
+  // dependent of the trace pass (see dg_apply_kernel)
+  template <int P, int NC, bool MASS, int BS, int MINB = (BS == 64 ? 6 : 1), bool ALIAS = false, int PDLM = 0>
+  static void run_cell(const DGProblem<T>* probs, int n, cudaStream_t s, int what, int* status) {
+    using S = DGShape<P, NC>;
+    int64_t n_blocks = 0;
+    const DGBatch<T> b = make_batch(probs, n, BS, n_blocks);
+    const size_t sm_trace = size_t(BS) * (S::US + S::QS) * sizeof(T);
+    // scalar problems: block-major traces (no shared memory in the trace pass)
+    constexpr bool BQ = NC == 1;
+    const size_t sm_apply = size_t(BS) * ((ALIAS ? 1 : 2) * S::US + S::QS) * sizeof(T);
+    static std::atomic<uint64_t> conf_t{0}, conf_a{0};
+    auto apply = dg_apply_kernel<P, NC, MASS, BS, T, MINB, ALIAS, BQ, (BQ ? PDLM : 0)>;
+    opt_in_smem(apply, sm_apply, conf_a);
+    if (what != 2) {
+      if constexpr (BQ) {
+        int64_t nbt = 0;
+        const DGBatch<T> bt = make_batch(probs, n, kQB, nbt);
+        if (trace_tma_ok<P>(probs, n)) run_trace_tma<P>(bt, nbt, s, status);
+        else dg_trace_blk_kernel<P, T><<<unsigned(nbt), kQB, 0, s>>>(bt, nbt);
+      } else {
+        opt_in_smem(dg_trace_kernel<P, NC, BS, T>, sm_trace, conf_t);
+        dg_trace_kernel<P, NC, BS, T><<<unsigned(n_blocks), BS, sm_trace, s>>>(b, n_blocks);
+      }
+    }
+    if (what == 1) return;
+    if (BQ && PDLM > 0 && what == 0) {
+      // the trace pass just launched on this stream is the only producer the
+      // apply pass may overlap: everything else it reads was complete before
+      // the trace pass started
+      cudaLaunchConfig_t lc = {};
+      lc.gridDim = dim3(unsigned(n_blocks));
+      lc.blockDim = dim3(BS);
+      lc.dynamicSmemBytes = sm_apply;
+      lc.stream = s;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      at[0].val.programmaticStreamSerializationAllowed = 1;
+      lc.attrs = at;
+      lc.numAttrs = 1;
+      SFEM_CUDA(cudaLaunchKernelEx(&lc, apply, b, n_blocks));
+    } else {
+      apply<<<unsigned(n_blocks), BS, sm_apply, s>>>(b, n_blocks);
+    }
+  }
+
+  // trace + apply with the cross-block neighbour data prefetched (scalar problems)
+  template <int P, int BS, int XCAP>
+  static void run_xp(const DGProblem<T>* probs, int n, cudaStream_t s, int what) {
+    using S = DGShape<P, 1>;
+    using O = gen::Ops<P>;
+    int64_t n_blocks = 0;
+    const DGBatch<T> b = make_batch(probs, n, BS, n_blocks);
+    const size_t sm_trace = size_t(BS) * (S::US + S::QS) * sizeof(T);
+    const size_t sm_apply = (size_t(BS) * (2 * S::US + S::QS) + size_t(XCAP) * (O::NF + O::NFQ)) * sizeof(T);
+    static std::atomic<uint64_t> conf_t{0}, conf_a{0};
+    auto trace = dg_trace_kernel<P, 1, BS, T>;
+    auto apply = dg_apply_xp_kernel<P, BS, XCAP, T>;
+    opt_in_smem(trace, sm_trace, conf_t);
+    opt_in_smem(apply, sm_apply, conf_a);
+    if (what != 2) trace<<<unsigned(n_blocks), BS, sm_trace, s>>>(b, n_blocks);
+    if (what != 1) apply<<<unsigned(n_blocks), BS, sm_apply, s>>>(b, n_blocks);
+  }
+
+  // phase-split scalar kernels (kernels_dg2.cuh): cross-block trace + apply
+  template <int P, bool MASS, int BS, int MINB, bool YS = false>
+  static void run_split(const DGProblem<T>* probs, int n, cudaStream_t s, int what) {
+    using S = DG2Shape<P, YS>;
+    int64_t n_blocks = 0;
+    const DGBatch<T> b = make_batch(probs, n, BS, n_blocks);
+    const size_t sm_trace = size_t(BS) * S::US * sizeof(T);
+    const size_t sm_apply = size_t(BS) * S::ELEMS * sizeof(T);
+    static std::atomic<uint64_t> conf_t{0}, conf_a{0};
+    auto trace = dg_trace_cross_kernel<P, BS, T>;
+    auto apply = dg_apply2_kernel<P, MASS, BS, T, MINB, YS>;
+    opt_in_smem(trace, sm_trace, conf_t);
+    opt_in_smem(apply, sm_apply, conf_a);
+    if (what != 2) trace<<<unsigned(n_blocks), BS, sm_trace, s>>>(b, n_blocks);
+    if (what != 1) apply<<<unsigned(n_blocks), BS, sm_apply, s>>>(b, n_blocks);
+  }
+
+  template <int P, int NC, bool MASS>
+  static void run_warp(const DGProblem<T>* probs, int n, cudaStream_t s, int what) {
+    using D = DG3<P, NC>;
+    int64_t n_blocks = 0;
+    const DGBatch<T> b = make_batch(probs, n, D::CELLS, n_blocks);
+    const size_t sm_trace = size_t(D::TRACE_ELEMS) * sizeof(T);
+    const size_t sm_apply = size_t(D::APPLY_ELEMS) * sizeof(T);
+    static std::atomic<uint64_t> conf_t{0}, conf_a{0};
+    opt_in_smem(dg3_trace_kernel<P, NC, T>, sm_trace, conf_t);
+    opt_in_smem(dg3_apply_kernel<P, NC, MASS, T>, sm_apply, conf_a);
+    if (what != 2) dg3_trace_kernel<P, NC, T><<<unsigned(n_blocks), D::THREADS, sm_trace, s>>>(b, n_blocks);
+    if (what != 1) dg3_apply_kernel<P, NC, MASS, T><<<unsigned(n_blocks), D::THREADS, sm_apply, s>>>(b, n_blocks);
+  }
+
+  template <int P, int NC, bool MASS>
+  static void run(const DGProblem<T>* probs, int n, cudaStream_t s, int what, int variant, int* status) {
+    if (what == 3) {
+      int64_t n_blocks = 0;
+      const DGBatch<T> b = make_batch(probs, n, 128, n_blocks);
+      dg_diagonal_kernel<P, NC, MASS, T><<<unsigned(n_blocks), 128, 0, s>>>(b, n_blocks);
+    } else if (variant == 1) {
+      // scalar problems: the apply pass loads its geometry and src rows while
+      // the trace pass finishes (B200, DG P3 FP64 32^3: 68.5 -> 64.5 us per vmult)
+      run_cell<P, NC, MASS, 128, 1, false, 1>(probs, n, s, what, status);
+    } else if (variant == 2) {
+      run_cell<P, NC, MASS, 64>(probs, n, s, what, status);
+    } else if (variant == 3) {
+      run_warp<P, NC, MASS>(probs, n, s, what);
+    } else if (variant == 5) {
+      // 64 cells per CTA, 5 CTAs per SM (up to 204 registers: no spills for P3)
+      run_cell<P, NC, MASS, 64, 5, false>(probs, n, s, what, status);
+    } else if (variant == 4) {
+      // 64 cells per CTA, results aliased onto the staged src rows (scalar
+      // problems), registers capped for 8 CTAs per SM; for scalar problems the
+      // cell term is computed while the trace pass finishes (B200, DG P3 FP32
+      // 32^3: 41.8 -> 38.0 us per vmult)
+      if (NC == 1) run_cell<P, NC, MASS, 64, 8, (NC == 1), 2>(probs, n, s, what, status);
+      else run_cell<P, NC, MASS, 64, 8, false>(probs, n, s, what, status);
+    } else if (variant == 7 || variant == 9) {
+      // phase-split scalar kernels (kernels_dg2.cuh): 7 results in registers,
+      // 64 cells x 5 CTAs per SM; 9 results in shared memory, 64 cells x 4
+      // CTAs (no spills); multi-component problems take the 128-cell form
+      if constexpr (NC == 1) {
+        if (variant == 7) run_split<P, MASS, 64, 5>(probs, n, s, what);
+        else run_split<P, MASS, 64, 4, true>(probs, n, s, what);
+      } else {
+        run_cell<P, NC, MASS, 128>(probs, n, s, what, status);
+      }
+    } else if (variant == 11) {
+      // 128 cells per CTA with the cross-block neighbour data prefetched into
+      // shared memory; multi-component and mass problems take the 128-cell form
+      if constexpr (NC == 1 && !MASS) run_xp<P, 128, 192>(probs, n, s, what);
+      else run_cell<P, NC, MASS, 128>(probs, n, s, what, status);
+    } else {
+      throw Error(FEM_ERR_ARG, "DG: kernel variant must be 0..5, 7, 9 or 11");
+    }
+    SFEM_CUDA(cudaGetLastError());
+  }
+};
+
+template <typename T>
+class DGBatchImpl final : public Batch {
+ public:
+  std::vector<DGOperator<T>*> ops;
+  // an operator listed more than once (several right-hand sides on one mesh)
+  // gets a trace scratch of its own for every repeat: the two passes of one
+  // launch must not share it between problems
+  std::vector<DevBuf<T>> extra_q;
+  std::vector<int> q_of;  // -1: the operator's own scratch, else index into extra_q
+  OpConfig cfg;
+  explicit DGBatchImpl(const std::vector<Operator*>& o) {
+    SFEM_REQUIRE(!o.empty() && int(o.size()) <= kMaxBatch, FEM_ERR_ARG, "batch: 1..40 operators");
+    cfg = o[0]->cfg;
+    for (auto* op : o) {
+      auto* d = dynamic_cast<DGOperator<T>*>(op);
+      SFEM_REQUIRE(d != nullptr, FEM_ERR_ARG, "batch: only DG/Helmholtz operators of one precision");
+      SFEM_REQUIRE(d->cfg.degree == cfg.degree && d->cfg.kind == cfg.kind &&
+                       d->cfg.n_components == cfg.n_components,
+                   FEM_ERR_ARG, "batch: operators must share kind, degree and components");
+      int repeat = -1;
+      for (auto* prev : ops)
+        if (prev == d) repeat = 0;
+      if (repeat == 0) {
+        extra_q.emplace_back(d->scratch_bytes() / sizeof(T));
+        repeat = int(extra_q.size()) - 1;
+      }
+      q_of.push_back(repeat);
+      ops.push_back(d);
+    }
+  }
+  void vmult(void* const* dst, const void* const* src, cudaStream_t s) override {
+    DGProblem<T> probs[kMaxBatch];
+    for (size_t i = 0; i < ops.size(); ++i) {
+      probs[i] = ops[i]->problem(src[i], dst[i]);
+      if (q_of[i] >= 0) probs[i].Q = extra_q[q_of[i]].p;
+    }
+    DGOperator<T>::launch_dg(cfg, probs, int(ops.size()), s, 0, ops[0]->d_status.p);
+  }
+  int variant() const override { return cfg.kernel_variant; }
+  void set_variant(int v) override {
+    SFEM_REQUIRE(v >= 0 && v <= 11 && v != 6 && v != 8 && v != 10, FEM_ERR_ARG,
+                 "batch: kernel variant must be 0..5, 7, 9 or 11");
+    cfg.kernel_variant = v;
+  }
+  TuneResult tune(int reps, bool use_cache) override {
+    TuneResult res;
+    res.us.assign(5, 0.0);
+    int64_t cells = 0;
+    for (auto* o : ops) cells += o->n_cells;
+    const std::string key = "batch" + std::to_string(ops.size()) + "," + tune_key(cfg, cells);
+    if (use_cache) {
+      const int v = tune_lookup(key);
+      if (v > 0) {
+        cfg.kernel_variant = v;
+        res.variant = v;
+        res.cached = true;
+        return res;
+      }
+    }
+    std::vector<DevBuf<T>> bufs;
+    std::vector<void*> d(ops.size());
+    std::vector<const void*> x(ops.size());
+    for (size_t i = 0; i < ops.size(); ++i) {
+      bufs.emplace_back(size_t(ops[i]->m));
+      bufs.emplace_back(size_t(ops[i]->m));
+      SFEM_CUDA(cudaMemset(bufs[2 * i].p, 0, sizeof(T) * ops[i]->m));
+    }
+    for (size_t i = 0; i < ops.size(); ++i) {
+      x[i] = bufs[2 * i].p;
+      d[i] = bufs[2 * i + 1].p;
+    }
+    cudaStream_t s = nullptr;
+    SFEM_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    const int keep = cfg.kernel_variant;
+    double best = 1e300;
+    try {
+      for (int v : tune_candidates(cfg)) {
+        cfg.kernel_variant = v;
+        const double us = time_launches([&](cudaStream_t st) { vmult(d.data(), x.data(), st); }, reps, s);
+        res.us[v - 1] = us;
+        if (us < best) {
+          best = us;
+          res.variant = v;
+        }
+      }
+    } catch (...) {
+      cfg.kernel_variant = keep;
+      cudaStreamDestroy(s);
+      throw;
+    }
+    cudaStreamDestroy(s);
+    cfg.kernel_variant = res.variant;
+    tune_store(key, res.variant, res.us);
+    return res;
+  }
+};
+
+}  // namespace
+
+template <typename T>
+std::unique_ptr<Operator> make_dg_operator(const Mesh& mesh, const OpConfig& cfg) {
+  return std::make_unique<DGOperator<T>>(mesh, cfg);
+}
+template <typename T>
+std::unique_ptr<Batch> make_dg_batch(const std::vector<Operator*>& ops) {
+  return std::make_unique<DGBatchImpl<T>>(ops);
+}
+
+}  // namespace sfem

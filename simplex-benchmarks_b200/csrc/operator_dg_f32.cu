@@ -1,0 +1,6 @@
+#include "operator_dg.cuh"
+
+namespace sfem {
+template std::unique_ptr<Operator> make_dg_operator<float>(const Mesh&, const OpConfig&);
+template std::unique_ptr<Batch> make_dg_batch<float>(const std::vector<Operator*>&);
+}  // namespace sfem
