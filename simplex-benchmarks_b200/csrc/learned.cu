@@ -12,6 +12,7 @@
 #include "learned.hpp"
 #include "mg.hpp"
 #include "mlp.cuh"
+#include "mlp_grad.cuh"
 #include "mlp_tc.cuh"
 #include "vector_kernels.cuh"
 
@@ -152,23 +153,55 @@ void LearnedSmoother::apply(const Operator& op, const void* r, void* z, cudaStre
   SFEM_CUDA(cudaGetLastError());
 }
 
-double LearnedSmoother::gradient(const float* X, const float* Y, int n, float* grad, cudaStream_t s) {
+namespace {
+// Samples per tile and CTAs of the gradient kernel: two CTAs of 256 threads fit
+// an SM.  Batches that 16-sample tiles spread over no more than one CTA per SM
+// take those (latency decides), larger ones 32-sample tiles (half the reads of
+// the weights per sample).
+struct GradPlan {
+  int spt, grid;
+};
+GradPlan mlp_grad_plan(int n, int sms) {
+  GradPlan p;
+  p.spt = (n + 15) / 16 <= sms ? 1 : 2;
+  p.grid = std::min((n + 16 * p.spt - 1) / (16 * p.spt), 2 * sms);
+  return p;
+}
+}  // namespace
+
+void LearnedSmoother::launch_gradient(const float* X, const float* Y, int n, float* grad, bool accumulate_loss,
+                                      cudaStream_t s) {
   static std::atomic<uint64_t> configured{0};
-  const int smem = 2 * NP * int(sizeof(float));
-  int dev = 0;
+  int dev = 0, sms = 0;
   SFEM_CUDA(cudaGetDevice(&dev));
   once_per_device(configured, dev, [&] {
-    SFEM_CUDA(cudaFuncSetAttribute(mlp_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    SFEM_CUDA(cudaFuncSetAttribute(mlp_grad_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   int(mlpg::Shape<1>::BYTES)));
+    SFEM_CUDA(cudaFuncSetAttribute(mlp_grad_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   int(mlpg::Shape<2>::BYTES)));
   });
+  SFEM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   SFEM_CUDA(cudaMemsetAsync(grad, 0, sizeof(float) * NP, s));
-  SFEM_CUDA(cudaMemsetAsync(loss_.p, 0, sizeof(float), s));
-  const int grid = std::min((n + 127) / 128, 148 * 2);
-  mlp_grad_kernel<<<grid, 128, smem, s>>>(n, X, Y, wb_.p, grad, loss_.p, 1.0f / float(n));
+  if (!accumulate_loss) SFEM_CUDA(cudaMemsetAsync(loss_.p, 0, sizeof(double), s));
+  const GradPlan p = mlp_grad_plan(n, sms);
+  const float inv = 1.0f / float(n);
+  if (p.spt == 1)
+    mlp_grad_kernel<1><<<p.grid, mlpg::THREADS, mlpg::Shape<1>::BYTES, s>>>(n, X, Y, wb_.p, grad, loss_.p, inv);
+  else
+    mlp_grad_kernel<2><<<p.grid, mlpg::THREADS, mlpg::Shape<2>::BYTES, s>>>(n, X, Y, wb_.p, grad, loss_.p, inv);
   SFEM_CUDA(cudaGetLastError());
-  float h = 0;
-  SFEM_CUDA(cudaMemcpyAsync(&h, loss_.p, sizeof(float), cudaMemcpyDeviceToHost, s));
+}
+
+double LearnedSmoother::read_loss(cudaStream_t s) {
+  double h = 0;
+  SFEM_CUDA(cudaMemcpyAsync(&h, loss_.p, sizeof(double), cudaMemcpyDeviceToHost, s));
   SFEM_CUDA(cudaStreamSynchronize(s));
-  return double(h) / n;
+  return h;
+}
+
+double LearnedSmoother::gradient(const float* X, const float* Y, int n, float* grad, cudaStream_t s) {
+  launch_gradient(X, Y, n, grad, false, s);
+  return read_loss(s);
 }
 
 void LearnedSmoother::forward(const float* X, float* O, int n, cudaStream_t s) {
@@ -208,11 +241,11 @@ TrainStats LearnedSmoother::train(const float* X, const float* Y, int n, int epo
     perm.upload(hp);
     gather_rows<<<unsigned((int64_t(n) * D::NIN + 255) / 256), 256, 0, s>>>(n, D::NIN, perm.p, X, Xp.p);
     gather_rows<<<unsigned((int64_t(n) * D::NOUT + 255) / 256), 256, 0, s>>>(n, D::NOUT, perm.p, Y, Yp.p);
-    double ep_loss = 0;
     int nb = 0;
     for (int off = 0; off + batch <= n || (off < n && nb == 0); off += batch) {
       const int cnt = std::min(batch, n - off);
-      ep_loss += gradient(Xp.p + int64_t(off) * D::NIN, Yp.p + int64_t(off) * D::NOUT, cnt, g_.p, s);
+      // the epoch's losses add up on the device, read back once per epoch
+      launch_gradient(Xp.p + int64_t(off) * D::NIN, Yp.p + int64_t(off) * D::NOUT, cnt, g_.p, nb > 0, s);
       ++adam_t_;
       const float c1 = 1.0f / (1.0f - std::pow(b1, float(adam_t_)));
       const float c2 = 1.0f / (1.0f - std::pow(b2, float(adam_t_)));
@@ -220,7 +253,7 @@ TrainStats LearnedSmoother::train(const float* X, const float* Y, int n, int epo
       round_weights(s);
       ++nb;
     }
-    ep_loss /= std::max(nb, 1);
+    const double ep_loss = read_loss(s) / std::max(nb, 1);
     if (ep == 0) st.loss_first = ep_loss;
     st.loss_last = ep_loss;
   }

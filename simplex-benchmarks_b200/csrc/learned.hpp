@@ -72,7 +72,11 @@ class LearnedSmoother {
   };
   Bound& bind(const Operator& op);
   void round_weights(cudaStream_t s);
-  DevBuf<float> w_, m_, v_, g_, loss_;
+  // gradient of the batch into grad and its loss (mean) into loss_, or added to it; no synchronisation
+  void launch_gradient(const float* X, const float* Y, int n, float* grad, bool accumulate_loss, cudaStream_t s);
+  double read_loss(cudaStream_t s);
+  DevBuf<float> w_, m_, v_, g_;
+  DevBuf<double> loss_;
   DevBuf<__nv_bfloat16> wb_;
   DevBuf<int> status_;
   bool tensor_cores_ = true;

@@ -22,14 +22,10 @@
 namespace sfem {
 
 // GELU in its tanh form, 0.5 x (1 + tanh(sqrt(2/pi) (x + 0.044715 x^3)))
-// (Hendrycks & Gimpel), and its derivative.
+// (Hendrycks & Gimpel); its derivative: gelu_both in mlp_grad.cuh.
 __device__ __forceinline__ float gelu(float x) {
   const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
   return 0.5f * x * (1.0f + tanhf(u));
-}
-__device__ __forceinline__ float gelu_grad(float x) {
-  const float t = tanhf(0.7978845608028654f * (x + 0.044715f * x * x * x));
-  return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * 0.7978845608028654f * (1.0f + 0.134145f * x * x);
 }
 // the same GELU with the hardware tanh approximation (tensor-core epilogues)
 // (6 instructions: u = x (c1 + c2 x^2), y = h + h tanh(u), h = x / 2)
@@ -52,7 +48,7 @@ __device__ __forceinline__ void mlp_load_weights(float* sw, const __nv_bfloat16*
   for (int i = threadIdx.x; i < MLPDims::NPARAM; i += blockDim.x) sw[i] = __bfloat162float(wb[i]);
 }
 
-// forward of one sample; a1/a2 are the pre-activations (kept for backward)
+// forward of one sample; a1/a2 are the pre-activations
 __device__ __forceinline__ void mlp_forward(const float* sw, const float (&x)[MLPDims::NIN], float (&a1)[MLPDims::NH],
                                             float (&a2)[MLPDims::NH], float (&o)[MLPDims::NOUT]) {
   using D = MLPDims;
@@ -121,79 +117,6 @@ __global__ void __launch_bounds__(128) mlp_smooth_kernel(int64_t n_cells, const 
     for (int i = 0; i < D::NR; ++i)
       if (g[i] >= 0) atomicAdd(z + g[i], T(scale * o[i] * winv[g[i]]));
   }
-}
-
-// One optimisation step's gradient over a batch: loss = mean_b ||o_b - y_b||^2.
-// X [n][29], Y [n][20]; grad (FP32, zeroed by the caller) accumulates dLoss/dW
-// (of the BF16 weights); loss_sum accumulates the summed loss.
-__global__ void __launch_bounds__(128) mlp_grad_kernel(int n, const float* __restrict__ X,
-                                                       const float* __restrict__ Y,
-                                                       const __nv_bfloat16* __restrict__ wb, float* __restrict__ grad,
-                                                       float* __restrict__ loss_sum, float inv_batch) {
-  using D = MLPDims;
-  extern __shared__ float smem_f[];  // 2 * NPARAM floats (dynamic, > 48 KB)
-  float* sw = smem_f;
-  float* sg = smem_f + D::NPARAM;
-  mlp_load_weights(sw, wb);
-  for (int i = threadIdx.x; i < D::NPARAM; i += blockDim.x) sg[i] = 0.0f;
-  __syncthreads();
-  float lsum = 0.0f;
-  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < n; b += gridDim.x * blockDim.x) {
-    float x[D::NIN], a1[D::NH], a2[D::NH], o[D::NOUT];
-#pragma unroll
-    for (int i = 0; i < D::NIN; ++i) x[i] = X[int64_t(b) * D::NIN + i];
-    mlp_forward(sw, x, a1, a2, o);
-    float dlo[D::NOUT];
-#pragma unroll
-    for (int j = 0; j < D::NOUT; ++j) {
-      const float d = o[j] - Y[int64_t(b) * D::NOUT + j];
-      lsum += d * d;
-      dlo[j] = 2.0f * d * inv_batch;
-    }
-    // layer 3
-    float h2[D::NH], dh[D::NH];
-#pragma unroll
-    for (int i = 0; i < D::NH; ++i) {
-      h2[i] = gelu(a2[i]);
-      dh[i] = 0.0f;
-    }
-    for (int j = 0; j < D::NOUT; ++j) {
-      atomicAdd(&sg[D::OFF_B3 + j], dlo[j]);
-#pragma unroll
-      for (int i = 0; i < D::NH; ++i) {
-        atomicAdd(&sg[D::OFF_W3 + j * D::NH + i], dlo[j] * h2[i]);
-        dh[i] = fmaf(sw[D::OFF_W3 + j * D::NH + i], dlo[j], dh[i]);
-      }
-    }
-    // layer 2
-#pragma unroll
-    for (int i = 0; i < D::NH; ++i) dh[i] *= gelu_grad(a2[i]);
-    float h1[D::NH], dh1[D::NH];
-#pragma unroll
-    for (int i = 0; i < D::NH; ++i) {
-      h1[i] = gelu(a1[i]);
-      dh1[i] = 0.0f;
-    }
-    for (int j = 0; j < D::NH; ++j) {
-      atomicAdd(&sg[D::OFF_B2 + j], dh[j]);
-#pragma unroll
-      for (int i = 0; i < D::NH; ++i) {
-        atomicAdd(&sg[D::OFF_W2 + j * D::NH + i], dh[j] * h1[i]);
-        dh1[i] = fmaf(sw[D::OFF_W2 + j * D::NH + i], dh[j], dh1[i]);
-      }
-    }
-    // layer 1
-    for (int j = 0; j < D::NH; ++j) {
-      const float d = dh1[j] * gelu_grad(a1[j]);
-      atomicAdd(&sg[D::OFF_B1 + j], d);
-#pragma unroll
-      for (int i = 0; i < D::NIN; ++i) atomicAdd(&sg[D::OFF_W1 + j * D::NIN + i], d * x[i]);
-    }
-  }
-  atomicAdd(loss_sum, lsum);
-  __syncthreads();
-  for (int i = threadIdx.x; i < D::NPARAM; i += blockDim.x)
-    if (sg[i] != 0.0f) atomicAdd(grad + i, sg[i]);
 }
 
 // forward only, for evaluation: O [n][20]

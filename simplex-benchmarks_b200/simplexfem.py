@@ -744,7 +744,7 @@ class MLP:
 
     def gradient(self, X, Y, stream=None):
         import torch
-        g = torch.zeros(mlp_n_params(), dtype=torch.float32, device="cuda")
+        g = torch.empty(mlp_n_params(), dtype=torch.float32, device="cuda")  # written whole by the call
         loss = C.c_double()
         check(lib().fem_mlp_gradient(self.handle, _ptr(X), _ptr(Y), X.shape[0], _ptr(g), C.byref(loss),
                                      _stream_ptr(stream)))
