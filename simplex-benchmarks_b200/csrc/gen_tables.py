@@ -8,8 +8,9 @@ this script:
 * ``ref_tables.h``   constexpr host/device tables (node lattice, nodal-gradient
   matrices, reference masses, face node lists, face masses, p-embeddings);
 * ``ref_kernels.cuh`` straight-line device functions that apply those matrices
-  with every structural zero removed and every +-1 folded, so that the cell and
-  face kernels run on compile-time constants only.
+  with every structural zero removed, every +-1 folded and the terms that
+  several rows share formed once (``shared_terms``), so that the cell and face
+  kernels run on compile-time constants only.
 
 Conventions (the DoF format every other part of the library relies on)
 -----------------------------------------------------------------------
@@ -37,11 +38,14 @@ product of traces equals 2|F| * (the reference-triangle integral), i.e. the
 tables already contain the factor 2 and kernels multiply by |F|.
 """
 from fractions import Fraction as Fr
-from itertools import product
+from itertools import combinations, product
 import math
 import os
+import random
 import sys
 
+# axis order of the six Kuhn tets of a hex (build_kuhn_mesh)
+KUHN = [(0, 1, 2), (0, 2, 1), (1, 0, 2), (1, 2, 0), (2, 0, 1), (2, 1, 0)]
 EDGES = [(0, 1), (0, 2), (0, 3), (1, 2), (1, 3), (2, 3)]
 
 
@@ -209,11 +213,13 @@ class Basis2:
             self.pts = [(Fr(1, 3), Fr(1, 3))]
             self.coef = [[Fr(1)]]
             self.mono = [(0, 0)]
+            self.lattice = [(0, 0, 0)]
             return
         bs = []
         for b0 in range(q, -1, -1):
             for b1 in range(q - b0, -1, -1):
                 bs.append((b0, b1, q - b0 - b1))
+        self.lattice = bs
         self.pts = [(Fr(b[1], q), Fr(b[2], q)) for b in bs]
         self.mono = monomials2(q)
         V = [[p[0] ** m[0] * p[1] ** m[1] for m in self.mono] for p in self.pts]
@@ -292,6 +298,12 @@ def build(pmax=3):
         EMB = None
         if p > 1:
             EMB = [[Bq.value(j, node_pos(Bp.nodes[i], p)) for j in range(KQ)] for i in range(K)]
+        # P_{p-1} face basis at the P_p face nodes: MFPQ = MFPP EMBF
+        EMBF = [[sum(c * pt[0] ** m[0] * pt[1] ** m[1] for c, m in zip(B2q.coef[j], B2q.mono)) for j in range(NFQ)]
+                for pt in B2p.pts]
+        for i in range(NF):
+            for j in range(NFQ):
+                assert MFPQ[i][j] == sum(MFPP[i][k] * EMBF[k][j] for k in range(NF))
         # consistency: D applied to the nodal interpolant of x_a gives 1 for d/dx_a
         for a in range(3):
             lin = [node_pos(nd, p)[a] for nd in Bp.nodes]
@@ -300,7 +312,7 @@ def build(pmax=3):
                     v = sum(D[b][m][i] * lin[i] for i in range(K))
                     assert v == (1 if a == b else 0)
         data[p] = dict(K=K, KQ=KQ, NF=NF, NFQ=NFQ, D=D, MQ=MQ, MP=MP, FN=FN, FNQ=FNQ,
-                       MFPP=MFPP, MFPQ=MFPQ, EMB=EMB,
+                       MFPP=MFPP, MFPQ=MFPQ, EMB=EMB, EMBF=EMBF, FLAT=B2p.lattice, FLATQ=B2q.lattice,
                        NODES=[node_pos(a, p) for a in Bp.nodes],
                        LATTICE=Bp.nodes, MONO=Bp.mono, COEF=Bp.coef)
     return data
@@ -383,55 +395,281 @@ def emit_matvec(lines, A, rows, cols, out_expr, in_expr, accumulate, transpose=F
     return nnz
 
 
+# ---- products with shared terms ---------------------------------------------------------------
+# A product y = A x of a fixed matrix is a straight-line program of multiply-adds.
+# Written row by row it costs one operation per non-zero.  Two rows that hold
+# the same two inputs in the same ratio can share that pair: t = x_i + r x_j is
+# one operation and saves one in every row that uses it.  Pairs are taken
+# greedily (most rows first, ties broken at random, the best of many orders
+# kept).  For the mass matrices, whose rows are a near-constant background plus
+# a few entries, the sums over symmetry classes of nodes (vertices, edges,
+# faces) are offered as extra inputs; face masses also in the even and odd
+# parts under the reflection that swaps two vertices, which decouple.
+# Operations per product (P1 / P2 / P3), row by row -> shared: gradient
+# 6/42/216 -> 3/24/113, its transpose 6/42/216 -> 6/36/145, gradient mass
+# 1/16/100 -> 1/11/55, cell mass 16/100/400 -> 10/55/153, face mass
+# 9/24/88 -> 7/22/66, face value-gradient mass 3/18/60 -> 3/14/43.
+# The generators print the counts.
+
+
+def row_cost(row):
+    return max(0, len(row) - (1 if any(abs(c) == 1 for c in row.values()) else 0))
+
+
+def share_pairs(rows, n_vars, rng):
+    """Greedy pair sharing; returns (definitions of the new variables, rows)."""
+    rows = [dict(r) for r in rows]
+    defs = []
+    while True:
+        found = {}
+        for k, r in enumerate(rows):
+            for a, b in combinations(sorted(r), 2):
+                found.setdefault((a, b, r[b] / r[a]), []).append(k)
+        most = max((len(v) for v in found.values()), default=0)
+        if most < 2:
+            return defs, rows
+        a, b, ratio = key = rng.choice([k for k, v in found.items() if len(v) == most])
+        for k in found[key]:
+            c = rows[k].pop(a)
+            rows[k].pop(b)
+            rows[k][n_vars + len(defs)] = c
+        defs.append({a: Fr(1), b: ratio})
+
+
+def sparse_rows(A):
+    return [{j: a for j, a in enumerate(r) if a != 0} for r in A]
+
+
+def with_class_sums(A, classes):
+    """Rows over the inputs and one extra input per class: the class's sum."""
+    n = len(A[0])
+    rows = []
+    for r in sparse_rows(A):
+        for k, cl in enumerate(classes):
+            vals = [r.get(j, Fr(0)) for j in cl]
+            c = max(sorted(set(vals)), key=vals.count)
+            if c == 0 or vals.count(c) < 2:
+                continue
+            for j in cl:
+                v = r.pop(j, Fr(0)) - c
+                if v != 0:
+                    r[j] = v
+            r[n + k] = c
+        rows.append(r)
+    return [{j: Fr(1) for j in cl} for cl in classes], rows
+
+
+def even_odd(A, perm_in, perm_out):
+    """Rows for the even and odd parts under a reflection A[po(i)][pi(j)] =
+    A[i][j]: extra inputs x_j +- x_pi(j), and for every pair of outputs its even
+    and odd half, recombined as (even + odd, even - odd)."""
+    n = len(A[0])
+    pairs = [(i, perm_in[i]) for i in range(n) if perm_in[i] > i]
+    fixed = [i for i in range(n) if perm_in[i] == i]
+    extra = [{i: Fr(1), j: Fr(s)} for i, j in pairs for s in (1, -1)]
+    rows, place = [], []
+    for r in range(len(A)):
+        q = perm_out[r]
+        if q < r:
+            continue
+        even = {i: A[r][i] for i in fixed if A[r][i] != 0}
+        odd = {}
+        for k, (i, j) in enumerate(pairs):
+            if A[r][i] + A[r][j] != 0:
+                even[n + 2 * k] = (A[r][i] + A[r][j]) / 2
+            if A[r][i] != A[r][j]:
+                odd[n + 2 * k + 1] = (A[r][i] - A[r][j]) / 2
+        rows.append(even)
+        if q == r:
+            place.append((r, len(rows) - 1, None))
+        else:
+            rows.append(odd)
+            place.append((r, len(rows) - 2, 1))
+            place.append((q, len(rows) - 2, -1))
+    return extra, rows, place
+
+
+def shared_terms(A, classes=(), reflections=(), tries=60, seed=0):
+    """The cheapest program found for y = A x: (cost, definitions, rows), variables
+    numbered inputs first, then definitions in order."""
+    n = len(A[0])
+    forms = [([], sparse_rows(A), None)]
+    for k in range(1, len(classes) + 1):
+        forms += [(*with_class_sums(A, sub), None) for sub in combinations(classes, k)]
+    forms += [even_odd(A, pi, po) for pi, po in reflections]
+    rng = random.Random(seed)
+    best = None
+    for extra, rows, place in forms:
+        for _ in range(tries):
+            defs, out = share_pairs(rows, n + len(extra), rng)
+            defs = extra + defs
+            if place is not None:
+                defs = defs + out
+                base = n + len(defs) - len(out)
+                at = [None] * len(A)
+                for r, k, sign in place:
+                    at[r] = {base + k: Fr(1)} if sign is None else {base + k: Fr(1), base + k + 1: Fr(sign)}
+                out = at
+            cost = sum(map(row_cost, defs)) + sum(map(row_cost, out))
+            if best is None or cost < best[0]:
+                best = (cost, defs, out)
+    check_program(A, best[1], best[2])
+    return best
+
+
+def check_program(A, defs, rows):
+    """The program is A, exactly."""
+    n = len(A[0])
+    val = [[Fr(int(i == j)) for j in range(n)] for i in range(n)]
+
+    def lin(r):
+        return [sum((c * val[v][j] for v, c in r.items()), Fr(0)) for j in range(n)]
+
+    for d in defs:
+        val.append(lin(d))
+    for r, want in zip(rows, A):
+        assert lin(r) == list(want)
+
+
+def emit_program(lines, program, n, out_expr, in_expr, accumulate):
+    """Emit the program; every definition right before its first use."""
+    _, defs, rows = program
+    done = set()
+
+    def name(v):
+        return in_expr(v) if v < n else f"t{v - n}"
+
+    def expr(r):
+        terms = sorted(r.items(), key=lambda vc: (abs(vc[1]) != 1, vc[1] < 0, vc[0]))
+        out = []
+        for v, c in terms:
+            if abs(c) == 1:
+                out.append(("+" if c > 0 else "-", name(v)))
+            else:
+                out.append(("+", f"T({fmt(c)}) * {name(v)}"))
+        return out
+
+    def join(terms):
+        s = terms[0][1] if terms[0][0] == "+" else f"-({terms[0][1]})"
+        return s + "".join(f" {sg} {t}" for sg, t in terms[1:])
+
+    def need(r):
+        for v in sorted(r):
+            if v >= n and v not in done:
+                done.add(v)
+                need(defs[v - n])
+                lines.append(f"  const T t{v - n} = {join(expr(defs[v - n]))};")
+
+    for k, r in enumerate(rows):
+        need(r)
+        if not r:
+            if not accumulate:
+                lines.append(f"  {out_expr(k)} = T(0);")
+        elif accumulate:
+            for sg, t in expr(r):
+                lines.append(f"  {out_expr(k)} {sg}= {t};")
+        else:
+            lines.append(f"  {out_expr(k)} = {join(expr(r))};")
+
+
+def node_classes(lattice, q):
+    """Nodes by kind (vertex, edge, face), kinds of at least two nodes."""
+    kinds = {}
+    for i, a in enumerate(lattice):
+        kinds.setdefault(sum(1 for x in a if x > 0), []).append(i)
+    return [v for _, v in sorted(kinds.items()) if len(v) > 1 and q > 0]
+
+
+def swap_perm(lattice, i, j):
+    def sw(a):
+        a = list(a)
+        a[i], a[j] = a[j], a[i]
+        return tuple(a)
+    return [lattice.index(sw(a)) for a in map(tuple, lattice)]
+
+
 def write_kernels(data, path):
     L = []
     L.append("// Generated by gen_tables.py from exact rational arithmetic. Do not edit.")
     L.append("// Straight-line applications of the reference matrices of ref_tables.h:")
-    L.append("// structural zeros are removed and +-1 entries folded, so cell and face")
-    L.append("// kernels issue only FMAs on compile-time constants.")
+    L.append("// structural zeros are removed, +-1 entries folded and terms that several rows")
+    L.append("// share formed once (t..), so cell and face kernels issue only additions and FMAs")
+    L.append("// on compile-time constants, about 0.6 of the operations of the plain rows for P3.")
     L.append("#pragma once\n")
     L.append("namespace sfem {\nnamespace gen {\n")
     stats = []
     for p, d in data.items():
         K, KQ, NF, NFQ = d["K"], d["KQ"], d["NF"], d["NFQ"]
+        kq = p - 1
+        lat, latq = list(d["LATTICE"]), (nodes(kq) if kq > 0 else [(0, 0, 0, 0)])
+        refl = (swap_perm(d["FLAT"], 0, 1), swap_perm(d["FLATQ"], 0, 1))
+
+        def fn(doc, sig, body):
+            L.append(f"// P{p}: {doc}")
+            L.append(f"template <typename T{', typename F' if 'F&&' in sig else ''}> __host__ __device__ __forceinline__ void {sig} {{")
+            L.extend(body)
+            L.append("}")
+
+        def product_fn(doc, sig, A, out_expr, in_expr, accumulate=False, classes=(), reflections=(), post=()):
+            prog = shared_terms(A, classes, reflections, tries=60 if len(A) < 16 else 30)
+            nonzeros = sum(1 for r in A for a in r if a != 0)
+            stats.append((p, sig.split("_P")[0], prog[0] + (sum(1 for r in prog[2] if any(abs(c) == 1 for c in r.values())) if accumulate else 0), nonzeros))
+            body = []
+            emit_program(body, prog, len(A[0]), out_expr, in_expr, accumulate)
+            fn(doc, sig, body + list(post))
+
         # nodal gradient: g[a][m] = sum_i D[a][m][i] u[i]
-        L.append(f"// P{p}: reference gradient in the P{p-1} nodal basis, g[a*{KQ}+m] = (D_a u)_m")
-        L.append(f"template <typename T> __host__ __device__ __forceinline__ void grad_P{p}(const T (&u)[{K}], T (&g)[{3*KQ}]) {{")
-        nz = 0
-        for a in range(3):
-            nz += emit_matvec(L, d["D"][a], KQ, K, lambda r, a=a: f"g[{a*KQ + r}]", lambda c: f"u[{c}]", False)
-        L.append("}")
-        stats.append((p, "grad", nz, 3 * KQ * K))
-        L.append(f"// P{p}: y += sum_a D_a^T h_a")
-        L.append(f"template <typename T> __host__ __device__ __forceinline__ void gradT_P{p}(const T (&h)[{3*KQ}], T (&y)[{K}]) {{")
+        DD = [row for a in range(3) for row in d["D"][a]]
+        product_fn(f"reference gradient in the P{p-1} nodal basis, g[a*{KQ}+m] = (D_a u)_m",
+                   f"grad_P{p}(const T (&u)[{K}], T (&g)[{3*KQ}])", DD, lambda r: f"g[{r}]", lambda c: f"u[{c}]")
         # y[i] += sum_{a,m} D[a][m][i] h[a*KQ+m]
-        DT = [[d["D"][a][m][i] for a in range(3) for m in range(KQ)] for i in range(K)]
-        nz = emit_matvec(L, DT, K, 3 * KQ, lambda r: f"y[{r}]", lambda c: f"h[{c}]", True)
-        L.append("}")
-        stats.append((p, "gradT", nz, 3 * KQ * K))
-        L.append(f"// P{p}: o = MQ w (reference-tet mass of P{p-1}), one gradient component")
-        L.append(f"template <typename T> __host__ __device__ __forceinline__ void massQ_P{p}(const T* w, T* o) {{")
-        emit_matvec(L, d["MQ"], KQ, KQ, lambda r: f"o[{r}]", lambda c: f"w[{c}]", False)
-        L.append("}")
-        L.append(f"// P{p}: y += MP u (reference-tet mass of P{p})")
-        L.append(f"template <typename T> __host__ __device__ __forceinline__ void massP_P{p}(const T* u, T s, T* y) {{")
-        # y += s * MP u  -> compute t = MP u then scale
-        L.append(f"  T t[{K}];")
-        emit_matvec(L, d["MP"], K, K, lambda r: f"t[{r}]", lambda c: f"u[{c}]", False)
-        L.append(f"  for (int i = 0; i < {K}; ++i) y[i] += s * t[i];")
-        L.append("}")
-        L.append(f"// P{p}: o = MFPP j (face mass P{p} x P{p}, factor 2 included)")
-        L.append(f"template <typename T> __host__ __device__ __forceinline__ void facePP_P{p}(const T* j, T* o) {{")
-        emit_matvec(L, d["MFPP"], NF, NF, lambda r: f"o[{r}]", lambda c: f"j[{c}]", False)
-        L.append("}")
-        L.append(f"// P{p}: o += MFPQ a (face mass P{p} x P{p-1})")
-        L.append(f"template <typename T> __host__ __device__ __forceinline__ void facePQ_P{p}(const T* a, T* o) {{")
-        emit_matvec(L, d["MFPQ"], NF, NFQ, lambda r: f"o[{r}]", lambda c: f"a[{c}]", True)
-        L.append("}")
-        L.append(f"// P{p}: o = MFPQ^T j (face mass P{p-1} x P{p})")
-        L.append(f"template <typename T> __host__ __device__ __forceinline__ void faceQP_P{p}(const T* j, T* o) {{")
-        emit_matvec(L, d["MFPQ"], NFQ, NF, lambda r: f"o[{r}]", lambda c: f"j[{c}]", False, transpose=True)
-        L.append("}")
+        product_fn("y += sum_a D_a^T h_a", f"gradT_P{p}(const T (&h)[{3*KQ}], T (&y)[{K}])",
+                   [list(c) for c in zip(*DD)], lambda r: f"y[{r}]", lambda c: f"h[{c}]", accumulate=True)
+        product_fn(f"o = MQ w (reference-tet mass of P{p-1}), one gradient component",
+                   f"massQ_P{p}(const T* w, T* o)", d["MQ"], lambda r: f"o[{r}]", lambda c: f"w[{c}]",
+                   classes=node_classes(latq, kq))
+        prog = shared_terms([list(c) for c in zip(*DD)], tries=60 if K < 16 else 30)
+        body = []
+        emit_program(body, prog, 3 * KQ, lambda r: f"y({r})", lambda c: f"h[{c}]", True)
+        fn("y(i) += (sum_a D_a^T h_a)_i", f"gradTInto_P{p}(const T (&h)[{3*KQ}], F&& y)", body)
+        # the same three row by row, for the CG kernels that run out of registers
+        # before they run out of arithmetic (see cg_local_apply)
+        body = []
+        for a in range(3):
+            emit_matvec(body, d["D"][a], KQ, K, lambda r, a=a: f"g[{a*KQ + r}]", lambda c: f"u[{c}]", False)
+        fn("grad, row by row", f"gradRows_P{p}(const T (&u)[{K}], T (&g)[{3*KQ}])", body)
+        body = []
+        emit_matvec(body, [list(c) for c in zip(*DD)], K, 3 * KQ, lambda r: f"y[{r}]", lambda c: f"h[{c}]", True)
+        fn("gradT, row by row", f"gradTRows_P{p}(const T (&h)[{3*KQ}], T (&y)[{K}])", body)
+        body = []
+        emit_matvec(body, [list(c) for c in zip(*DD)], K, 3 * KQ, lambda r: f"y({r})", lambda c: f"h[{c}]", True)
+        fn("gradTInto, row by row", f"gradTRowsInto_P{p}(const T (&h)[{3*KQ}], F&& y)", body)
+        body = []
+        emit_matvec(body, d["MQ"], KQ, KQ, lambda r: f"o[{r}]", lambda c: f"w[{c}]", False)
+        fn("massQ, row by row", f"massQRows_P{p}(const T* w, T* o)", body)
+        # y += s * MP u: t = MP u, then scaled
+        prog = shared_terms(d["MP"], node_classes(lat, p), [(swap_perm(lat, 0, 1),) * 2] if p > 1 else (), tries=10)
+        stats.append((p, "massP", prog[0], K * K))
+        body = [f"  T o[{K}];"]
+        emit_program(body, prog, K, lambda r: f"o[{r}]", lambda c: f"u[{c}]", False)
+        body.append(f"  for (int i = 0; i < {K}; ++i) y[i] += s * o[i];")
+        fn(f"y += s MP u (reference-tet mass of P{p})", f"massP_P{p}(const T* u, T s, T* y)", body)
+        fcl = node_classes(d["FLAT"], p)
+        product_fn(f"o = MFPP j (face mass P{p} x P{p}, factor 2 included)", f"facePP_P{p}(const T* j, T* o)", d["MFPP"],
+                   lambda r: f"o[{r}]", lambda c: f"j[{c}]", classes=fcl, reflections=[(refl[0], refl[0])])
+        fqcl = node_classes(d["FLATQ"], p - 1)
+        product_fn(f"o += MFPQ a (face mass P{p} x P{p-1})", f"facePQ_P{p}(const T* a, T* o)", d["MFPQ"],
+                   lambda r: f"o[{r}]", lambda c: f"a[{c}]", accumulate=True, classes=fqcl)
+        product_fn(f"o = MFPQ^T j (face mass P{p-1} x P{p})", f"faceQP_P{p}(const T* j, T* o)",
+                   [list(c) for c in zip(*d["MFPQ"])], lambda r: f"o[{r}]", lambda c: f"j[{c}]", classes=fcl)
+        # the face terms of the DG apply: the factors 1/4 of the averages and of the
+        # gradient test are in the matrices
+        quarter = [[-a / 4 for a in r] for r in d["MFPQ"]]
+        product_fn("o(i) += (-1/4 MFPQ a)_i", f"faceFlux_P{p}(const T* a, F&& o)", quarter,
+                   lambda r: f"o({r})", lambda c: f"a[{c}]", accumulate=True, classes=fqcl)
+        product_fn(f"o = -1/4 MFPQ^T j from t = MFPP j (MFPQ = MFPP E, E the P{p-1} face basis at the P{p} nodes)",
+                   f"faceTest_P{p}(const T* t, T* o)", [[-a / 4 for a in c] for c in zip(*d["EMBF"])],
+                   lambda r: f"o[{r}]", lambda c: f"t[{c}]")
         L.append("")
     # single-row functions for warp-split kernels: a switch on the row index
     # that folds away once the caller's loops are unrolled
@@ -501,6 +739,13 @@ def write_kernels(data, path):
         L.append(f"  static constexpr int K = {K}, KQ = {KQ}, NF = {NF}, NFQ = {NFQ};")
         L.append(f"  template <class T> static __device__ __forceinline__ void grad(const T (&u)[{K}], T (&g)[{3*KQ}]) {{ grad_P{p}(u, g); }}")
         L.append(f"  template <class T> static __device__ __forceinline__ void gradT(const T (&h)[{3*KQ}], T (&y)[{K}]) {{ gradT_P{p}(h, y); }}")
+        L.append(f"  template <class T> static __device__ __forceinline__ void gradRows(const T (&u)[{K}], T (&g)[{3*KQ}]) {{ gradRows_P{p}(u, g); }}")
+        L.append(f"  template <class T> static __device__ __forceinline__ void gradTRows(const T (&h)[{3*KQ}], T (&y)[{K}]) {{ gradTRows_P{p}(h, y); }}")
+        L.append(f"  template <class T, class F> static __device__ __forceinline__ void gradTInto(const T (&h)[{3*KQ}], F&& y) {{ gradTInto_P{p}(h, y); }}")
+        L.append(f"  template <class T, class F> static __device__ __forceinline__ void gradTRowsInto(const T (&h)[{3*KQ}], F&& y) {{ gradTRowsInto_P{p}(h, y); }}")
+        L.append(f"  template <class T> static __device__ __forceinline__ void massQRows(const T* w, T* o) {{ massQRows_P{p}(w, o); }}")
+        L.append(f"  template <class T, class F> static __device__ __forceinline__ void faceFlux(const T* a, F&& o) {{ faceFlux_P{p}(a, o); }}")
+        L.append(f"  template <class T> static __device__ __forceinline__ void faceTest(const T* t, T* o) {{ faceTest_P{p}(t, o); }}")
         L.append(f"  template <class T> static __device__ __forceinline__ void massQ(const T* w, T* o) {{ massQ_P{p}(w, o); }}")
         L.append(f"  template <class T> static __device__ __forceinline__ void massP(const T* u, T s, T* y) {{ massP_P{p}(u, s, y); }}")
         L.append(f"  template <class T> static __device__ __forceinline__ void facePP(const T* j, T* o) {{ facePP_P{p}(j, o); }}")
@@ -515,6 +760,18 @@ def write_kernels(data, path):
         L.append(f"  static __host__ __device__ __forceinline__ constexpr int faceq_pos(int f, int m) {{ return faceq_pos_P{p}(f, m); }}")
         cases = " ".join(f"case {f*NF+i}: return {d['FN'][f][i]};" for f in range(4) for i in range(NF))
         L.append(f"  static __host__ __device__ __forceinline__ constexpr int fn(int f, int i) {{ switch (f * {NF} + i) {{ {cases} }} return 0; }}")
+        # Kuhn hex: lattice offset (x, y, z in 0..p) of node i of tet q.  Tet q walks
+        # the hex edges in axis order KUHN[q], which is also the order of its
+        # (ascending) vertices.
+        hexn = []
+        for q in range(6):
+            for a in d["LATTICE"]:
+                off = [0, 0, 0]
+                for s, axis in enumerate(KUHN[q]):
+                    off[axis] = sum(a[s + 1:])
+                hexn.append(off[0] + (p + 1) * (off[1] + (p + 1) * off[2]))
+        cases = " ".join(f"case {k}: return {v};" for k, v in enumerate(hexn))
+        L.append(f"  static __host__ __device__ __forceinline__ constexpr int hex_node(int q, int i) {{ switch (q * {K} + i) {{ {cases} }} return 0; }}")
         cases = " ".join(f"case {f*NFQ+i}: return {d['FNQ'][f][i]};" for f in range(4) for i in range(NFQ))
         L.append(f"  static __host__ __device__ __forceinline__ constexpr int fnq(int f, int m) {{ switch (f * {NFQ} + m) {{ {cases} }} return 0; }}")
         L.append("};")
@@ -531,7 +788,7 @@ def main():
     write_tables(data, os.path.join(here, "ref_tables.h"))
     stats = write_kernels(data, os.path.join(here, "ref_kernels.cuh"))
     for s in stats:
-        print("P%d %-6s nonzeros %4d of %4d" % s)
+        print("P%d %-10s %4d operations for %4d non-zeros" % s)
 
 
 if __name__ == "__main__":

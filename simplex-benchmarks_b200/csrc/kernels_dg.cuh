@@ -138,23 +138,23 @@ __device__ __forceinline__ void face_cf(const T (&G)[6], int f, T (&cf)[3]) {
   }
 }
 
-// coalesced copy of `rows` rows of N contiguous values into padded rows.  A
-// full block from a 16-byte aligned source takes 16-byte loads, all issued
-// before the first shared-memory store (N / (16 / sizeof(T)) per thread in
-// flight); other blocks copy value by value.
-template <int N, int S, int BS, typename T>
-__device__ __forceinline__ void stage_in(T* __restrict__ sm, const T* __restrict__ g, int rows) {
+// coalesced copy of `rows` rows of N contiguous values into padded rows by
+// THREADS threads.  A full block of BS rows from a 16-byte aligned source takes
+// 16-byte loads, all issued before the first shared-memory store (N BS / THREADS
+// / (16 / sizeof(T)) per thread in flight); other blocks copy value by value.
+template <int N, int S, int BS, int THREADS, typename T>
+__device__ __forceinline__ void copy_rows_in(T* __restrict__ sm, const T* __restrict__ g, int rows) {
   constexpr int V = 16 / int(sizeof(T));  // values per 16-byte load
-  if constexpr (N % V == 0) {
+  if constexpr (BS * N % (V * THREADS) == 0) {
     if (rows == BS && (reinterpret_cast<uintptr_t>(g) & 15u) == 0) {
-      constexpr int PER = N / V;  // 16-byte loads per thread
+      constexpr int PER = BS * N / (V * THREADS);  // 16-byte loads per thread
       uint4 w[PER];
 #pragma unroll
-      for (int k = 0; k < PER; ++k) w[k] = __ldg(reinterpret_cast<const uint4*>(g) + k * BS + threadIdx.x);
+      for (int k = 0; k < PER; ++k) w[k] = __ldg(reinterpret_cast<const uint4*>(g) + k * THREADS + threadIdx.x);
 #pragma unroll
       for (int k = 0; k < PER; ++k) {
         const T* v = reinterpret_cast<const T*>(&w[k]);
-        const int e0 = (k * BS + threadIdx.x) * V;
+        const int e0 = (k * THREADS + threadIdx.x) * V;
 #pragma unroll
         for (int q = 0; q < V; ++q) sm[((e0 + q) / N) * S + ((e0 + q) % N)] = v[q];
       }
@@ -162,29 +162,38 @@ __device__ __forceinline__ void stage_in(T* __restrict__ sm, const T* __restrict
     }
   }
   const int total = rows * N;
-  for (int e = threadIdx.x; e < total; e += BS) sm[(e / N) * S + (e % N)] = __ldg(g + e);
+  for (int e = threadIdx.x; e < total; e += THREADS) sm[(e / N) * S + (e % N)] = __ldg(g + e);
 }
 // the reverse copy; full blocks to a 16-byte aligned destination take 16-byte stores
-template <int N, int S, int BS, typename T>
-__device__ __forceinline__ void stage_out(T* __restrict__ g, const T* __restrict__ sm, int rows) {
+template <int N, int S, int BS, int THREADS, typename T>
+__device__ __forceinline__ void copy_rows_out(T* __restrict__ g, const T* __restrict__ sm, int rows) {
   constexpr int V = 16 / int(sizeof(T));
-  if constexpr (N % V == 0) {
+  if constexpr (BS * N % (V * THREADS) == 0) {
     if (rows == BS && (reinterpret_cast<uintptr_t>(g) & 15u) == 0) {
-      constexpr int PER = N / V;
+      constexpr int PER = BS * N / (V * THREADS);
 #pragma unroll
       for (int k = 0; k < PER; ++k) {
-        const int e0 = (k * BS + threadIdx.x) * V;
+        const int e0 = (k * THREADS + threadIdx.x) * V;
         uint4 w;
         T* v = reinterpret_cast<T*>(&w);
 #pragma unroll
         for (int q = 0; q < V; ++q) v[q] = sm[((e0 + q) / N) * S + ((e0 + q) % N)];
-        reinterpret_cast<uint4*>(g)[k * BS + threadIdx.x] = w;
+        reinterpret_cast<uint4*>(g)[k * THREADS + threadIdx.x] = w;
       }
       return;
     }
   }
   const int total = rows * N;
-  for (int e = threadIdx.x; e < total; e += BS) g[e] = sm[(e / N) * S + (e % N)];
+  for (int e = threadIdx.x; e < total; e += THREADS) g[e] = sm[(e / N) * S + (e % N)];
+}
+// the same by the CTA's BS threads
+template <int N, int S, int BS, typename T>
+__device__ __forceinline__ void stage_in(T* __restrict__ sm, const T* __restrict__ g, int rows) {
+  copy_rows_in<N, S, BS, BS>(sm, g, rows);
+}
+template <int N, int S, int BS, typename T>
+__device__ __forceinline__ void stage_out(T* __restrict__ g, const T* __restrict__ sm, int rows) {
+  copy_rows_out<N, S, BS, BS>(g, sm, rows);
 }
 
 // ---- block-major traces (scalar problems) ------------------------------------------------------
@@ -473,6 +482,31 @@ __device__ __forceinline__ void dg_cell_term(const T* u, const T (&G)[6], T md, 
   if (MASS) O::massP(uu, md, y);
 }
 
+// Terms of one face from the jump j and the difference dq of the two outward
+// normal derivatives (scaled by 2|F|): value test y += sigma|F| MFPP j - 1/4
+// MFPQ dq, gradient test h_a += -1/4 cf_a MFPQ^T j.  MFPQ^T j comes from MFPP j
+// (the P_{p-1} face functions are P_p face functions too).
+template <int P, typename T>
+__device__ __forceinline__ void face_apply(int f, const T (&j)[gen::Ops<P>::NF], const T (&dq)[gen::Ops<P>::NFQ],
+                                           T sf, const T (&cf)[3], T (&h)[3 * gen::Ops<P>::KQ],
+                                           T (&y)[gen::Ops<P>::K]) {
+  using O = gen::Ops<P>;
+  constexpr int KQ = O::KQ, NF = O::NF, NFQ = O::NFQ;
+  T t[NF], r[NFQ];
+  O::facePP(j, t);
+  O::faceTest(t, r);
+#pragma unroll
+  for (int i = 0; i < NF; ++i) y[O::fn(f, i)] += sf * t[i];
+  O::faceFlux(dq, [&](int i) -> T& { return y[O::fn(f, i)]; });
+#pragma unroll
+  for (int m = 0; m < NFQ; ++m) {
+    const int nq = O::fnq(f, m);
+    h[nq] += cf[0] * r[m];
+    h[KQ + nq] += cf[1] * r[m];
+    h[2 * KQ + nq] += cf[2] * r[m];
+  }
+}
+
 // The four faces' terms of one component added to the cell term (h, y),
 // then y += D^T h.  Arguments as for dg_cell_component.
 template <int P, int NC, bool HAVE_NB, typename T, bool XS = false, bool BQ = false, int BSQ = 1>
@@ -484,7 +518,7 @@ __device__ __forceinline__ void dg_face_terms(const DGProblem<T>& pr, int64_t c0
                                               const T* xs = nullptr, const int (*slot)[4] = nullptr) {
   using O = gen::Ops<P>;
   using S = DGShape<P, NC>;
-  constexpr int K = O::K, KQ = O::KQ, NF = O::NF, NFQ = O::NFQ;
+  constexpr int K = O::K, NF = O::NF, NFQ = O::NFQ;
   static_assert(!BQ || NC == 1, "block-major traces are for scalar problems");
   constexpr int QST = BQ ? BSQ : 1;  // stride of a cell's consecutive traces in shared memory
   const T* u = us + comp * K;
@@ -493,14 +527,16 @@ __device__ __forceinline__ void dg_face_terms(const DGProblem<T>& pr, int64_t c0
     T cf[3];
     face_cf(G, f, cf);
     const T* qm = qs + (BQ ? f * NFQ * BSQ : (f * NC + comp) * NFQ);
-    T j[NF], avg[NFQ];
+    // jump of the values and difference of the outward normal derivatives; the
+    // averages' 1/4 and signs are in faceFlux and faceTest
+    T j[NF], dq[NFQ];
     if (nb[f] >= 0) {
       if (XS && (*slot)[f] >= 0) {
         const T* xn = xs + (*slot)[f] * (NF + NFQ);
 #pragma unroll
         for (int i = 0; i < NF; ++i) j[i] = u[O::fn(f, i)] - xn[i];
 #pragma unroll
-        for (int m = 0; m < NFQ; ++m) avg[m] = T(0.25) * (qm[m * QST] - xn[NF + m]);
+        for (int m = 0; m < NFQ; ++m) dq[m] = qm[m * QST] - xn[NF + m];
       } else if (HAVE_NB) {
         const int64_t lc = int64_t(nb[f]) - c0;
         const T* un;
@@ -519,41 +555,21 @@ __device__ __forceinline__ void dg_face_terms(const DGProblem<T>& pr, int64_t c0
 #pragma unroll
         for (int i = 0; i < NF; ++i) j[i] = u[O::fn(f, i)] - un[O::fn_runtime(nbf[f], i)];
 #pragma unroll
-        for (int m = 0; m < NFQ; ++m) avg[m] = T(0.25) * (qm[m * QST] - qn[m * qns]);
+        for (int m = 0; m < NFQ; ++m) dq[m] = qm[m * QST] - qn[m * qns];
       } else {
 #pragma unroll
         for (int i = 0; i < NF; ++i) j[i] = u[O::fn(f, i)];
 #pragma unroll
-        for (int m = 0; m < NFQ; ++m) avg[m] = T(0.25) * qm[m * QST];
+        for (int m = 0; m < NFQ; ++m) dq[m] = qm[m * QST];
       }
     } else {
       // boundary face: u+ = -u-, d_n u+ = d_n u-
 #pragma unroll
       for (int i = 0; i < NF; ++i) j[i] = T(2) * u[O::fn(f, i)];
 #pragma unroll
-      for (int m = 0; m < NFQ; ++m) avg[m] = T(0.5) * qm[m * QST];
+      for (int m = 0; m < NFQ; ++m) dq[m] = T(2) * qm[m * QST];
     }
-    // value test: sigma|F| MFPP j - MFPQ avg
-    T t[NF];
-    O::facePP(j, t);
-#pragma unroll
-    for (int i = 0; i < NF; ++i) t[i] *= sf[f];
-#pragma unroll
-    for (int m = 0; m < NFQ; ++m) avg[m] = -avg[m];
-    O::facePQ(avg, t);
-#pragma unroll
-    for (int i = 0; i < NF; ++i) y[O::fn(f, i)] += t[i];
-    // gradient test: h_a += -1/4 cf_a MFQP j
-    T r[NFQ];
-    O::faceQP(j, r);
-#pragma unroll
-    for (int m = 0; m < NFQ; ++m) {
-      const int nq = O::fnq(f, m);
-      const T rm = T(-0.25) * r[m];
-      h[nq] += cf[0] * rm;
-      h[KQ + nq] += cf[1] * rm;
-      h[2 * KQ + nq] += cf[2] * rm;
-    }
+    face_apply<P>(f, j, dq, sf[f], cf, h, y);
   }
   O::gradT(h, y);
 }
