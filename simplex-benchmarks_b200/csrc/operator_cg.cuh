@@ -12,6 +12,7 @@
 #include "kernels_dg.cuh"
 #include "op_shapes.hpp"
 #include "operator.hpp"
+#include "operator_cg_block.hpp"
 #include "operator_parts.hpp"
 
 namespace sfem {
@@ -90,6 +91,9 @@ class CGOperator final : public Operator {
     if (clear && v) SFEM_CUDA(cudaMemset(d_status.p, 0, sizeof(int)));
     return v;
   }
+
+  // 4 x 4 x 4-hex blocks of cg_block_kernel; empty on meshes that are no Kuhn boxes
+  CGBlocks<T, 1> blocks;
 
   // cube-block tables of cg_cube_kernel (blocks of 64 hexes = 384 tets)
   DevBuf<int16_t> d_tmapv, d_cslot8[3];
@@ -511,6 +515,7 @@ class CGOperator final : public Operator {
     d_constrained.upload(cl);
     build_hex_tables(mesh, dofs, geo);
     build_cube_tables(dofs);
+    blocks.build(mesh, cfg.degree, dofs.cell_dofs, dofs.constrained, geo);
     if (cfg.weak_bc) build_weak_boundary(mesh);
     d_status.alloc(1);
     SFEM_CUDA(cudaMemset(d_status.p, 0, sizeof(int)));
@@ -629,11 +634,27 @@ class CGOperator final : public Operator {
     SFEM_CUDA(cudaGetLastError());
   }
 
+  // Block form (cg_block_kernel) or thread-per-tet cube kernel, where both apply.
+  // P1 and P2: always the block form.  P3 FP32: the block form once its blocks fill
+  // the SMs more than half (64 threads walk a whole block, 15 us: 32^3 15.8 against
+  // 17.4 us, but 24^3 15.6 against 10.4 us) or where there are no whole cubes.  P3
+  // FP64 (two resident CTAs of 64 threads): never (64^3 177 against 143 us).
+  bool use_blocks() const {
+    if (cfg.degree <= 2) return true;
+    return sizeof(T) == 4 && (!cube_NB || blocks.n_blocks >= 400);
+  }
+  // Variant 0: forms 3 (blocks or cubes) and 1 (thread per cell), the latter on
+  // meshes with fewer blocks than SMs, where most SMs would idle (P2 FP64 16^3 5.0
+  // against 7.8 us, 24^3 equal, 32^3 13.9 against 8.9 us), and for P3 FP64 without
+  // whole cubes (37 x 41 x 35 hexes: 41.5 us, per hex 49.5 us).
+  int default_variant() const {
+    const bool cubes = cube_NB && n_blocks >= 2 * 148;
+    if (cfg.degree <= 2) return blocks.n_blocks >= 148 ? 3 : 1;
+    if (cubes || (sizeof(T) == 4 && blocks.n_blocks >= 148)) return 3;
+    return 1;
+  }
+
   void apply_cells(const T* x, T* d, cudaStream_t s) {
-    // default (variant 0), measured on B200: P1 per cube in FP64 and per hex
-    // in FP32, P2 per cube, P3 per cube in FP32 and per cell in FP64; per cell on meshes too small to give
-    // every SM two cubes (or two CTAs of hexes), where the coarser forms
-    // leave SMs idle
     int v = cfg.kernel_variant;
     if (v == 8) {
       // TF32 tensor cores per cube; per cell (variant 4) without whole cubes
@@ -654,18 +675,16 @@ class CGOperator final : public Operator {
       launch_tc_cell(x, d, s);
       return;
     }
-    if (v == 0) {
-      constexpr int64_t kFill = 2 * 148;
-      // measured on B200: P3 FP64 64^3 cube 171 against 190 us per cell
-      v = cfg.degree == 1 ? (sizeof(T) == 8 ? 3 : 2) : 3;
-      if (v == 3 && n_blocks < kFill) v = 2;
-      if (v == 2 && n_hex < kFill * kHexBS) v = 1;
-    }
-    // cube reduce schedule: variants 5, 6, 7 pick one; variant 3 takes the
-    // one measured fastest on B200 (FP64 P1 and P2: bank-scheduled with
-    // uniform steps, 144 against 157 us and 380 against 380-413 us on 128^3;
+    if (v == 0) v = default_variant();
+    // variant 3: the block form where it is the faster one, else the cube kernel;
+    // cube reduce schedule: variants 5, 6, 7 pick one; variant 3 takes the one
+    // measured fastest on B200 (FP64 P1 and P2: bank-scheduled with uniform steps;
     // FP32 and P3: contribution order)
     int sched = v >= 5 ? v - 5 : (sizeof(T) == 8 && cfg.degree <= 2 ? 1 : 0);
+    if (v == 3 && blocks.n_blocks && use_blocks()) {
+      blocks.launch(cfg.degree, x, d, d_constrained.n, d_constrained.p, s);
+      return;
+    }
     if (v >= 5) v = 3;
     if (v == 3 && cube_NB) {
       switch (cfg.degree) {
@@ -742,7 +761,7 @@ class CGOperator final : public Operator {
 // (index 3 g + comp), as the reference's components-batched CG operator
 // (CG/components_batched/application.cc:778-1611, FESystem of dim
 // FE_SimplexP).  Homogeneous Dirichlet on every component of the boundary
-// nodes.  Cell kernel only.
+// nodes.  Thread per cell, or cg_block_kernel on Kuhn boxes.
 template <typename T>
 class CGVectorOperator final : public Operator {
  public:
@@ -752,6 +771,7 @@ class CGVectorOperator final : public Operator {
   DevBuf<int32_t> d_constrained;  // constrained vector indices
   int64_t n_nodes = 0;
   std::vector<int32_t> node_dofs;  // [n_cells][K]
+  CGBlocks<T, NC> blocks;          // 4 x 4 x 4-hex blocks (Kuhn boxes)
 
   CGVectorOperator(const Mesh& mesh, const OpConfig& c) {
     cfg = c;
@@ -792,6 +812,7 @@ class CGVectorOperator final : public Operator {
     }
     d_geo.upload(geo);
     d_constrained.upload(cl);
+    blocks.build(mesh, cfg.degree, dofs.cell_dofs, dofs.constrained, geo);
   }
 
   void vmult(void* dst, const void* src, cudaStream_t s) override {
@@ -804,6 +825,11 @@ class CGVectorOperator final : public Operator {
     const T* x = static_cast<const T*>(src);
     if (phase == 1) {
       SFEM_CUDA(cudaMemsetAsync(d, 0, sizeof(T) * m, s));
+      return;
+    }
+    // P3 FP64: the block form is slower than a thread per cell (48^3 392 against 226 us)
+    if (cfg.kernel_variant == 0 && blocks.n_blocks >= 148 && (cfg.degree <= 2 || sizeof(T) == 4)) {
+      blocks.launch(cfg.degree, x, d, d_constrained.n, d_constrained.p, s);
       return;
     }
     const unsigned grid = blocks_for(std::max<int64_t>(n_cells, int64_t(d_constrained.n)), 128);
