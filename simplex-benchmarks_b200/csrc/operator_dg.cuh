@@ -10,6 +10,7 @@
 #include "kernels_dg.cuh"
 #include "kernels_dg2.cuh"
 #include "kernels_dg3.cuh"
+#include "kernels_dg_fused.cuh"
 #include "op_shapes.hpp"
 #include "operator.hpp"
 #include "operator_parts.hpp"
@@ -25,6 +26,10 @@ class DGOperator final : public Operator {
   DevBuf<T> d_geo;      // [6 + 4 + (mass?1:0)][n_cells]
   DevBuf<int32_t> d_nb; // [4][n_cells]
   DevBuf<int8_t> d_nbf; // [4][n_cells]
+  // P1 and P2, single-pass form (kernels_dg_fused.cuh)
+  DevBuf<unsigned char> d_fgeo;  // geometry by blocks of cells
+  DevBuf<int32_t> d_ext_begin, d_ext;  // outer neighbours of every block
+  int n_ext = 0;            // most of a block
   DevBuf<T> d_Q;        // published face normal derivatives: [n_cells][4][NC][NFQ], or block-major
                         // (scalar problems, 1-thread-per-cell forms), for whole 128-cell blocks
   DevBuf<int> d_status; // timeouts of the bounded waits in the bulk-copy trace pass
@@ -103,9 +108,69 @@ class DGOperator final : public Operator {
       }
     d_nb.upload(nb);
     d_nbf.upload(nbf);
+    if (p <= 2) build_fused(mesh, geo);
     d_Q.alloc(size_t((n_cells + kQB - 1) / kQB * kQB) * 4 * cfg.n_components * nfq_of(p));
     d_status.alloc(1);
     SFEM_CUDA(cudaMemset(d_status.p, 0, sizeof(int)));
+  }
+
+  static int fused_block(int nc) { return nc == 1 ? dg_fused_cells<1>() : dg_fused_cells<3>(); }
+
+  void build_fused(const Mesh& mesh, const std::vector<T>& geo) {
+    const int64_t BS = fused_block(cfg.n_components), nblk = (n_cells + BS - 1) / BS;
+    const int NG = has_mass ? 23 : 22;  // FusedShape
+    const size_t block_bytes = size_t(NG) * BS * sizeof(T) + 4 * BS * sizeof(uint16_t);
+    std::vector<unsigned char> fg(block_bytes * nblk, 0);
+    std::vector<std::vector<int32_t>> outer(nblk);
+#pragma omp parallel for schedule(static)
+    for (int64_t b = 0; b < nblk; ++b) {
+      const int64_t c0 = b * BS, c1 = std::min(n_cells, c0 + BS);
+      T* g = reinterpret_cast<T*>(fg.data() + b * block_bytes);
+      uint16_t* code = reinterpret_cast<uint16_t*>(g + NG * BS);
+      std::fill(code, code + 4 * BS, kBoundary);
+      std::vector<int32_t>& ex = outer[b];
+      for (int64_t cc = c0; cc < c1; ++cc)
+        for (int f = 0; f < 4; ++f) {
+          const int32_t nbc = mesh.nb[4 * cc + f];
+          if (nbc >= 0 && (nbc < c0 || nbc >= c1)) ex.push_back(nbc);
+        }
+      std::sort(ex.begin(), ex.end());
+      ex.erase(std::unique(ex.begin(), ex.end()), ex.end());
+      for (int64_t cc = c0; cc < c1; ++cc) {
+        for (int k = 0; k < 10; ++k) g[k * BS + cc - c0] = geo[size_t(k) * n_cells + cc];
+        if (has_mass) g[22 * BS + cc - c0] = geo[size_t(10) * n_cells + cc];
+        for (int f = 0; f < 4; ++f) {
+          // J^-1 (2|F| n) of the neighbour on its side of the face, as the barycentric
+          // weights of the three face vertices (own values on the boundary, unread)
+          const int32_t nbc = mesh.nb[4 * cc + f];
+          const int64_t o = nbc >= 0 ? nbc : cc;
+          const int of = nbc >= 0 ? mesh.nbf[4 * cc + f] : f;
+          double G[6], w[4] = {0, 0, 0, 0};
+          metric(cell_geometry(mesh, o), G);
+          const double M[3][3] = {{G[0], G[3], G[4]}, {G[3], G[1], G[5]}, {G[4], G[5], G[2]}};
+          for (int a = 0; a < 3; ++a) {
+            w[a + 1] = of == 0 ? M[a][0] + M[a][1] + M[a][2] : -M[a][of - 1];
+            w[0] -= w[a + 1];
+          }
+          for (int v = 0, k = 0; v < 4; ++v)
+            if (v != of) g[(10 + 3 * f + k++) * BS + cc - c0] = T(w[v]);
+          if (nbc < 0) continue;
+          const int64_t row = nbc >= c0 && nbc < c1
+                                  ? nbc - c0
+                                  : BS + (std::lower_bound(ex.begin(), ex.end(), nbc) - ex.begin());
+          code[f * BS + cc - c0] = uint16_t(row << 2 | of);
+        }
+      }
+    }
+    std::vector<int32_t> begin(nblk + 1, 0), ext;
+    for (int64_t b = 0; b < nblk; ++b) {
+      n_ext = std::max(n_ext, int(outer[b].size()));
+      ext.insert(ext.end(), outer[b].begin(), outer[b].end());
+      begin[b + 1] = int32_t(ext.size());
+    }
+    d_ext_begin.upload(begin);
+    d_fgeo.upload(fg);
+    d_ext.upload(ext);
   }
 
   int status(bool clear) override {
@@ -120,6 +185,10 @@ class DGOperator final : public Operator {
     pr.geo = d_geo.p;
     pr.nb = d_nb.p;
     pr.nbf = d_nbf.p;
+    pr.fgeo = d_fgeo.p;
+    pr.ext_begin = d_ext_begin.p;
+    pr.ext = d_ext.p;
+    pr.n_ext = n_ext;
     pr.src = static_cast<const T*>(src);
     pr.dst = static_cast<T*>(dst);
     pr.Q = d_Q.p;
@@ -185,7 +254,8 @@ class DGOperator final : public Operator {
     throw Error(FEM_ERR_ARG, "DG: unsupported degree/components combination");
   }
 
-  // kernel forms: 1 thread per cell, 128 cells per CTA; 2 thread per cell, 64
+  // kernel forms: 1 thread per cell, 128 cells per CTA (P1 and P2: one pass with a
+  // thread per cell and component); 2 thread per cell, 64
   // cells per CTA; 3 warp roles, 32 cells per CTA
   // (measured on B200: scalar P3 runs best register-capped at 64 cells per CTA,
   // the 3-component forms at 128 cells per CTA)
@@ -296,6 +366,22 @@ class DGOperator final : public Operator {
     }
   }
 
+  // P1 and P2 in one pass (kernels_dg_fused.cuh)
+  template <int P, int NC, bool MASS>
+  static void run_fused(const DGProblem<T>* probs, int n, cudaStream_t s) {
+    constexpr int BS = dg_fused_cells<NC>();
+    using S = FusedShape<P, NC, MASS, BS, T>;
+    int64_t n_blocks = 0;
+    const DGBatch<T> b = make_batch(probs, n, BS, n_blocks);
+    int rows = BS;
+    for (int i = 0; i < n; ++i) rows = std::max(rows, BS + probs[i].n_ext);
+    static std::atomic<uint64_t> conf{0};
+    auto kern = dg_fused_kernel<P, NC, MASS, BS, T, dg_fused_min_ctas<P, NC, T>()>;
+    // at most BS cells with four outer neighbours each
+    opt_in_smem(kern, S::bytes(5 * BS), conf);
+    kern<<<unsigned(n_blocks), BS * NC, S::bytes(rows), s>>>(b);
+  }
+
   // trace + apply with the cross-block neighbour data prefetched (scalar problems)
   template <int P, int BS, int XCAP>
   static void run_xp(const DGProblem<T>* probs, int n, cudaStream_t s, int what) {
@@ -351,6 +437,10 @@ class DGOperator final : public Operator {
       int64_t n_blocks = 0;
       const DGBatch<T> b = make_batch(probs, n, 128, n_blocks);
       dg_diagonal_kernel<P, NC, MASS, T><<<unsigned(n_blocks), 128, 0, s>>>(b, n_blocks);
+    } else if (variant == 1 && P <= 2 && what == 0) {
+      // P1 and P2: one pass (B200, 45 x 38 x 31 hexes: see kernels_dg_fused.cuh); the
+      // two passes below are what vmult_phase runs
+      if constexpr (P <= 2) run_fused<P, NC, MASS>(probs, n, s);
     } else if (variant == 1) {
       // scalar problems: the apply pass loads its geometry and src rows while
       // the trace pass finishes (B200, DG P3 FP64 32^3: 68.5 -> 64.5 us per vmult)
