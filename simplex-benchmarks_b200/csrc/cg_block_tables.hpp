@@ -14,6 +14,7 @@ namespace sfem {
 struct CGBlockTables {
   int64_t n_blocks = 0;         // 0: the mesh is no Kuhn box (or too large for the codes)
   std::vector<int32_t> codes;   // [n_blocks][NBP]
+  std::vector<uint8_t> upper;   // [n_blocks]: bit d set if the box goes on in direction d
   std::vector<int32_t> cell;    // [n_blocks][6][64]: cell of tet q of hex t, -1 where the box ends
 };
 
@@ -136,7 +137,12 @@ inline CGBlockTables build_cg_block_tables(const Mesh& mesh, int p, const std::v
     const int q = kuhn_tet(mesh, c, h);
     if (q < 0) return CGBlockTables{};
     int32_t& b = id[h[0] / 4 + int64_t(nb[0]) * (h[1] / 4 + int64_t(nb[1]) * (h[2] / 4))];
-    if (b < 0) b = int32_t(blocks++);
+    if (b < 0) {
+      b = int32_t(blocks++);
+      uint8_t up = 0;
+      for (int d = 0; d < 3; ++d) up |= uint8_t((h[d] / 4 + 1 < nb[d]) << d);
+      T.upper.push_back(up);
+    }
     where[c] = b;
     place[c] = int16_t(64 * q + (h[0] & 3) + 4 * (h[1] & 3) + 16 * (h[2] & 3));
   }

@@ -15,6 +15,7 @@
 #pragma once
 #include <cstdint>
 
+#include "pdl.cuh"
 #include "ref_kernels.cuh"
 
 namespace sfem {
@@ -102,21 +103,24 @@ __global__ void __launch_bounds__(128, MINB) cg_cell_kernel(int64_t n_cells, con
                                                       const int32_t* __restrict__ constrained) {
   using O = gen::Ops<P>;
   const int64_t c = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  // the operator's own tables before the wait for src and dst
+  int32_t idx[O::K];
+  T G[6];
+  if (c < n_cells) {
+#pragma unroll
+    for (int i = 0; i < O::K; ++i) idx[i] = __ldg(dofs + i * n_cells + c);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) G[k] = __ldg(geo + k * n_cells + c);
+  }
+  pdl_enter();
   if (c < n_constrained) {
     const int32_t i = constrained[c];
     dst[i] = src[i];
   }
   if (c >= n_cells) return;
-  int32_t idx[O::K];
   T u[O::K];
 #pragma unroll
-  for (int i = 0; i < O::K; ++i) {
-    idx[i] = __ldg(dofs + i * n_cells + c);
-    u[i] = idx[i] >= 0 ? __ldg(src + idx[i]) : T(0);
-  }
-  T G[6];
-#pragma unroll
-  for (int k = 0; k < 6; ++k) G[k] = __ldg(geo + k * n_cells + c);
+  for (int i = 0; i < O::K; ++i) u[i] = idx[i] >= 0 ? __ldg(src + idx[i]) : T(0);
   T y[O::K];
   cg_local_apply<P>(G, u, y);
 #pragma unroll
@@ -138,17 +142,21 @@ __global__ void __launch_bounds__(128) cg_cell_vec_kernel(int64_t n_cells, const
                                                           const int32_t* __restrict__ constrained) {
   using O = gen::Ops<P>;
   const int64_t c = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  // the operator's own tables before the wait for src and dst
+  int32_t idx[O::K];
+  T G[6];
+  if (c < n_cells) {
+#pragma unroll
+    for (int i = 0; i < O::K; ++i) idx[i] = __ldg(dofs + i * n_cells + c);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) G[k] = __ldg(geo + k * n_cells + c);
+  }
+  pdl_enter();
   if (c < n_constrained) {
     const int32_t i = constrained[c];
     dst[i] = src[i];
   }
   if (c >= n_cells) return;
-  int32_t idx[O::K];
-#pragma unroll
-  for (int i = 0; i < O::K; ++i) idx[i] = __ldg(dofs + i * n_cells + c);
-  T G[6];
-#pragma unroll
-  for (int k = 0; k < 6; ++k) G[k] = __ldg(geo + k * n_cells + c);
 #pragma unroll 1
   for (int comp = 0; comp < NC; ++comp) {
     T u[O::K], y[O::K];
@@ -411,6 +419,7 @@ __global__ void __launch_bounds__(384, cube_min_ctas<P, T>())
   T* yr = ubuf + 2 * NB;                    // [384][KP], then the zero slots
   const int t = threadIdx.x;
   if (t < (sizeof(T) == 8 ? 16 : 32)) yr[384 * KP + t] = T(0);
+  pdl_enter();
   const int64_t stride = gridDim.x;
   const int64_t n_cells = n_blocks * 384;
   for (int64_t i = blockIdx.x * int64_t(384) + t; i < n_constrained; i += stride * 384) {

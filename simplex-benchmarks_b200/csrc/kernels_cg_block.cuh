@@ -99,10 +99,6 @@ __global__ void __launch_bounds__(64, MINB)
   T* yb = ub + NC * S::LATP;                                   // [NC][LATP] sums
   const int t = threadIdx.x;
   const int64_t stride = gridDim.x;
-  for (int64_t i = blockIdx.x * int64_t(64) + t; i < n_constrained; i += stride * 64) {
-    const int32_t g = constrained[i];
-    dst[g] = src[g];
-  }
   for (int e = t; e < NBP / 8; e += 64)
     reinterpret_cast<uint4*>(sp)[e] = __ldg(reinterpret_cast<const uint4*>(pos) + e);
   auto issue_codes = [&](int64_t b, int slot) {
@@ -150,12 +146,17 @@ __global__ void __launch_bounds__(64, MINB)
 
   int64_t b = blockIdx.x;
   issue_codes(b, 0);
+  T G[2][6];
+  if (b < n_blocks) load_geo(b, 0, G[0]);
+  pdl_enter();  // the operator's own tables are on their way; src and dst from here on
+  for (int64_t i = blockIdx.x * int64_t(64) + t; i < n_constrained; i += stride * 64) {
+    const int32_t g = constrained[i];
+    dst[g] = src[g];
+  }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
   issue_gather(b, 0);
   issue_codes(b + stride, 1);
-  T G[2][6];
-  if (b < n_blocks) load_geo(b, 0, G[0]);
   int cur = 0;  // ring slot of block b's codes
   for (; b < n_blocks; b += stride) {
     const int nxt = cur + 1 == S::RING ? 0 : cur + 1;

@@ -47,6 +47,7 @@
 #include <cstdint>
 
 #include "kernels_cg.cuh"
+#include "pdl.cuh"
 #include "ref_kernels.cuh"
 #include "tcgen05.cuh"
 
@@ -117,15 +118,11 @@ __device__ __forceinline__ void cp_async_elem(T* smem, const T* gmem) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
-// Programmatic dependent launch (sm_90 and later).  The trace pass lets the
-// apply pass of the same vmult launch while it still runs; the apply pass
-// does the work that does not read the traces (its geometry, neighbour ids,
-// src rows, optionally the cell term) and then waits for the whole trace grid
-// - its completion and the visibility of its stores - before it reads Q.  A
-// kernel launched without the programmatic-serialization attribute returns
-// from the wait at once.
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The trace pass lets the apply pass of the same vmult launch while it still runs
+// (pdl.cuh); the apply pass does the work that does not read the traces (its
+// geometry, neighbour ids, src rows, optionally the cell term) and then waits for
+// the whole trace grid before it reads Q.  src is complete by then: the trace
+// pass triggers its dependents only after its own wait.
 
 // J^-1 (2|F_f| n_f) for local face f
 template <typename T>
@@ -261,7 +258,7 @@ __global__ void __launch_bounds__(kQB) dg_trace_blk_kernel(const __grid_constant
                                                            int64_t n_blocks) {
   using O = gen::Ops<P>;
   constexpr int K = O::K, KQ = O::KQ, NFQ = O::NFQ, QN = 4 * NFQ;
-  pdl_trigger();
+  pdl_enter();
   for (int64_t blk = blockIdx.x; blk < n_blocks; blk += gridDim.x) {
     const int pi = find_problem(batch, blk);
     const DGProblem<T>& pr = batch.p[pi];
@@ -356,9 +353,11 @@ __global__ void __launch_bounds__(kQB) dg_trace_tma_kernel(const __grid_constant
   if (t == 0) {
     for (int s = 0; s < NS; ++s) mbar_init(bar0 + 8 * s, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  pdl_enter();
+  if (t == 0) {
     for (int64_t k = 0; k < NS && k < mine; ++k) issue(k);
   }
-  pdl_trigger();
   __syncthreads();
   int64_t done = 0;  // blocks whose stage wait completed
   bool ok = true;
@@ -661,7 +660,7 @@ __global__ void __launch_bounds__(BS, MINB) dg_apply_kernel(const __grid_constan
       __syncthreads();  // src rows staged
       T h[3 * O::KQ], y[O::K];
       if (t < nloc) dg_cell_term<P, MASS>(su + t * S::US, d.G, d.md, h, y);
-      pdl_wait();
+      pdl_enter();
       stage_q_blk<S::QN, BS>(sq, pr.Q, c0, nloc);
       __syncthreads();
       if (t < nloc)
@@ -676,7 +675,7 @@ __global__ void __launch_bounds__(BS, MINB) dg_apply_kernel(const __grid_constan
       stage_out<S::U, S::US, BS>(pr.dst + c0 * S::U, sy, nloc);
       continue;
     }
-    if constexpr (PDLM == 1) pdl_wait();
+    if constexpr (PDLM == 1) pdl_enter();
     if constexpr (BQ) stage_q_blk<S::QN, BS>(sq, pr.Q, c0, nloc);
     else stage_in<S::QN, S::QS, BS>(sq, pr.Q + c0 * S::QN, nloc);
     __syncthreads();

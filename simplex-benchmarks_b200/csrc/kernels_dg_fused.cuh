@@ -229,6 +229,7 @@ __global__ void __launch_bounds__(BS* NC, MINB) dg_fused_kernel(const __grid_con
     const unsigned char* g = pr.fgeo + lb * S::GEO;
     for (int e = t; e < S::GEO / 16; e += THREADS) cp_async_bytes<16>(smem_raw + 16 * e, g + 16 * e);
   }
+  pdl_enter();  // the vectors' producer
   if ((reinterpret_cast<uintptr_t>(pr.src) & uintptr_t(S::CB - 1)) == 0) {
     const T* own = pr.src + c0 * S::U;
     for (int e = t; e < nloc * S::CH; e += THREADS)

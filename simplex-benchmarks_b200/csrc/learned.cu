@@ -331,7 +331,7 @@ TrainStats LearnedSmoother::generate_and_train(const TrainParams& p) {
         SFEM_CUDA(cudaMemsetAsync(x.p, 0, sizeof(double) * m, s));
         if (k > 0) solver.solve(x.p, b.p, 1e-30, k, s);
         op->vmult(r.p, x.p, s);
-        vec_residual<double><<<grid_for(m), 256, 0, s>>>(m, b.p, r.p, r.p);  // r = b - A x
+        vec_residual<double><<<grid_for(m), 256, 0, s>>>(m, b.p, r.p, r.p, nullptr, 0, 0);  // r = b - A x
         SFEM_CUDA(cudaMemcpyAsync(e.p, xs.p, sizeof(double) * m, cudaMemcpyDeviceToDevice, s));
         vec_axpby<double><<<grid_for(m), 256, 0, s>>>(m, -1.0, x.p, 1.0, e.p);  // e = x* - x
         // what the smoother has to remove: the part left after the (accurate)

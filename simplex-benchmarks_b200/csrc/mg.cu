@@ -19,7 +19,9 @@
 #include <vector>
 
 #include "learned.hpp"
+#include "cg_block_tables.hpp"
 #include "mg.hpp"
+#include "mg_block_transfer.cuh"
 #include "ref_tables.h"
 #include "vector_kernels.cuh"
 
@@ -47,6 +49,7 @@ __global__ void transfer_prolongate_add(int64_t nf, int Kf, int Kc, const int32_
                                         const double* __restrict__ mats, const int32_t* __restrict__ fdofs,
                                         const int32_t* __restrict__ cdofs, int64_t nc, const T* __restrict__ xc,
                                         T* __restrict__ xf) {
+  pdl_enter();
   const int64_t c = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (c >= nf) return;
   const uint32_t ow = owner[c];
@@ -74,6 +77,7 @@ __global__ void transfer_restrict_add(int64_t nf, int Kf, int Kc, const int32_t*
                                       const double* __restrict__ mats, const int32_t* __restrict__ fdofs,
                                       const int32_t* __restrict__ cdofs, int64_t nc, const T* __restrict__ xf,
                                       T* __restrict__ xc) {
+  pdl_enter();
   const int64_t c = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (c >= nf) return;
   const uint32_t ow = owner[c];
@@ -107,6 +111,7 @@ __global__ void __launch_bounds__(128) transfer_prolongate_add_k(int64_t nf, con
                                                                  const int32_t* __restrict__ fdofs,
                                                                  const int32_t* __restrict__ cdofs, int64_t nc,
                                                                  const T* __restrict__ xc, T* __restrict__ xf) {
+  pdl_enter();
   const int64_t c = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (c >= nf) return;
   const uint32_t ow = __ldg(owner + c);
@@ -139,6 +144,7 @@ __global__ void __launch_bounds__(128) transfer_restrict_add_k(int64_t nf, const
                                                                const int32_t* __restrict__ fdofs,
                                                                const int32_t* __restrict__ cdofs, int64_t nc,
                                                                const T* __restrict__ xf, T* __restrict__ xc) {
+  pdl_enter();
   const int64_t c = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (c >= nf) return;
   const uint32_t ow = __ldg(owner + c);
@@ -180,6 +186,7 @@ __global__ void __launch_bounds__(128) transfer_p_prolongate_k(int64_t n, const 
                                                                const int32_t* __restrict__ fdofs,
                                                                const int32_t* __restrict__ cdofs,
                                                                const T* __restrict__ xc, T* __restrict__ xf) {
+  pdl_enter();
   const int64_t c = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (c >= n) return;
   const uint32_t ow = __ldg(owner + c);
@@ -208,6 +215,7 @@ __global__ void __launch_bounds__(128) transfer_p_restrict_k(int64_t n, const ui
                                                              const int32_t* __restrict__ fdofs,
                                                              const int32_t* __restrict__ cdofs,
                                                              const T* __restrict__ xf, T* __restrict__ xc) {
+  pdl_enter();
   const int64_t c = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (c >= n) return;
   const uint32_t ow = __ldg(owner + c);
@@ -238,6 +246,7 @@ __global__ void __launch_bounds__(128) transfer_p_restrict_k(int64_t n, const ui
 template <typename T>
 __global__ void dg_p_prolongate_add(int64_t n, int Kf, int Kc, const double* __restrict__ emb,
                                     const T* __restrict__ xc, T* __restrict__ xf) {
+  pdl_enter();
   const int64_t c = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (c >= n) return;
   double xl[20];
@@ -252,6 +261,7 @@ __global__ void dg_p_prolongate_add(int64_t n, int Kf, int Kc, const double* __r
 template <typename T>
 __global__ void dg_p_restrict_add(int64_t n, int Kf, int Kc, const double* __restrict__ emb,
                                   const T* __restrict__ xf, T* __restrict__ xc) {
+  pdl_enter();
   const int64_t c = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (c >= n) return;
   double rl[20];
@@ -267,25 +277,40 @@ __global__ void dg_p_restrict_add(int64_t n, int Kf, int Kc, const double* __res
 // (DG/cells_batched/application_phc.cc:3476-3552): prolongation copies the
 // continuous nodal values into every cell (0 at constrained nodes),
 // restriction sums the cells' values back (its transpose).
+// A CTA's 128 cells' rows go through shared memory: the DG side is read and
+// written in runs, the table and the CG values per thread (16^3 P3: 15 -> 4 us).
+constexpr int kCRow = 21;  // padded row (K <= 20): odd, so a thread's row is conflict-free
 template <typename T>
-__global__ void c_prolongate_add(int64_t n, int K, const int32_t* __restrict__ cdofs, const T* __restrict__ xcg,
-                                 T* __restrict__ xdg) {
-  const int64_t c = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (c >= n) return;
-  for (int i = 0; i < K; ++i) {
-    const int32_t g = cdofs[i * n + c];
-    if (g >= 0) xdg[c * K + i] += xcg[g];
-  }
+__global__ void __launch_bounds__(128) c_prolongate_add(int64_t n, int K, const int32_t* __restrict__ cdofs,
+                                                        const T* __restrict__ xcg, T* __restrict__ xdg) {
+  __shared__ T s[128 * kCRow];
+  pdl_enter();
+  const int64_t c0 = blockIdx.x * int64_t(128), c = c0 + threadIdx.x;
+  if (c < n)
+    for (int i = 0; i < K; ++i) {
+      const int32_t g = __ldg(cdofs + i * n + c);
+      s[threadIdx.x * kCRow + i] = g >= 0 ? xcg[g] : T(0);
+    }
+  __syncthreads();
+  const int total = int(n - c0 < 128 ? n - c0 : 128) * K;
+  T* out = xdg + c0 * K;
+  for (int e = threadIdx.x; e < total; e += 128) out[e] += s[(e / K) * kCRow + e % K];
 }
 
 template <typename T>
-__global__ void c_restrict_add(int64_t n, int K, const int32_t* __restrict__ cdofs, const T* __restrict__ xdg,
-                               T* __restrict__ xcg) {
-  const int64_t c = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+__global__ void __launch_bounds__(128) c_restrict_add(int64_t n, int K, const int32_t* __restrict__ cdofs,
+                                                      const T* __restrict__ xdg, T* __restrict__ xcg) {
+  __shared__ T s[128 * kCRow];
+  pdl_enter();
+  const int64_t c0 = blockIdx.x * int64_t(128), c = c0 + threadIdx.x;
+  const int total = int(n - c0 < 128 ? n - c0 : 128) * K;
+  const T* in = xdg + c0 * K;
+  for (int e = threadIdx.x; e < total; e += 128) s[(e / K) * kCRow + e % K] = in[e];
+  __syncthreads();
   if (c >= n) return;
   for (int i = 0; i < K; ++i) {
-    const int32_t g = cdofs[i * n + c];
-    if (g >= 0) atomicAdd(xcg + g, xdg[c * K + i]);
+    const int32_t g = __ldg(cdofs + i * n + c);
+    if (g >= 0) atomicAdd(xcg + g, s[threadIdx.x * kCRow + i]);
   }
 }
 
@@ -502,6 +527,15 @@ double tridiag_max_eig(const std::vector<double>& a, const std::vector<double>& 
   return hi;
 }
 
+// Whether the readers of a product's result clear it for the next product instead
+// of a fill before it: one launch less, which decides on small vectors.  On large
+// ones the fill right before the product is better, since its zeros are still in
+// L2 when the operator adds into them (B200, CG P3 FP32: 7.2M values, smoothing
+// step 143 us with a fill, 156 us cleared in passing; equal at 0.9M values).
+bool clear_in_passing(const Operator& op) {
+  return op.needs_zero() && size_t(op.m) * op.elem_size() <= (size_t(8) << 20);
+}
+
 template <typename T>
 class MultigridImpl final : public Multigrid {
  public:
@@ -515,6 +549,7 @@ class MultigridImpl final : public Multigrid {
     double lmax = 0, lmin = 0;
     int degree = 1;
     int hexes = 1;
+    bool clear_t = false;  // t is zero between products (see product())
     // transfer from level-1 (absent on level 0)
     int Kf = 0, Kc = 0;
     DevBuf<int32_t> parent;
@@ -522,17 +557,23 @@ class MultigridImpl final : public Multigrid {
     DevBuf<uint32_t> owner;
     DevBuf<double> mats;
     std::vector<double> mats_host;  // p-transfers: the embedding matrix as a kernel parameter
+    // p-transfers by blocks (mg_block_transfer.cuh)
+    bool by_blocks = false;
+    DevBuf<uint16_t> bt_ent, bt_list, bt_order;
+    DevBuf<uint8_t> bt_hi;
+    DevBuf<int32_t> bt_start;
+    BlockWeights bt_w{};
+    int bt_grid[2] = {0, 0};  // persistent CTAs: prolongation, restriction
   };
   std::vector<std::unique_ptr<Mesh>> meshes_;  // owned h-level meshes
   std::vector<Level> levels_;
   DevBuf<double> coarse_inv_;
   int coarse_n_ = 0;
-  DevBuf<double> d_in_, d_out_, partial_, scal_, step_;
+  DevBuf<double> partial_, scal_, step_;
   DevBuf<T> cc_rhs_, cc_y_;  // coarse-correction work vectors (level below the finest)
   cudaGraph_t graph_[2] = {nullptr, nullptr};      // [0] Chebyshev, [1] learned finest level
   cudaGraphExec_t exec_[2] = {nullptr, nullptr};
   cudaStream_t cap_stream_ = nullptr;
-  int64_t fine_m_ = 0;
   LearnedSmoother* learned_ = nullptr;
   bool use_learned_ = false;
   bool fallback_enabled_ = false;
@@ -546,7 +587,6 @@ class MultigridImpl final : public Multigrid {
     const Mesh& mf = *fine.mesh;
     SFEM_REQUIRE(mf.structured, FEM_ERR_ARG,
                  "multigrid: the h-levels need a Kuhn box mesh (fem_mesh_create), not a mesh from arrays");
-    fine_m_ = fine.m;
     // number of h-levels
     int H = 0;
     {
@@ -601,6 +641,7 @@ class MultigridImpl final : public Multigrid {
       cfg.weak_bc = prm.weak_cg_levels && L.kind == FEM_CG;
       L.op = make_operator(*L.mesh, cfg);
       const int64_t m = L.op->m;
+      L.clear_t = clear_in_passing(*L.op);
       L.inv_diag.alloc(m);
       L.x.alloc(m);
       L.b.alloc(m);
@@ -640,16 +681,18 @@ class MultigridImpl final : public Multigrid {
       F.mat_id.upload(th.mat_id);
       F.owner.upload(th.owner);
       F.mats.upload(th.mats);
-      if (F.mesh == Cl.mesh) F.mats_host = th.mats;
+      if (F.mesh == Cl.mesh) {
+        F.mats_host = th.mats;
+        build_block_transfer(F, Cl);
+      }
     }
-    partial_.alloc(kReduceBlocks);
+    partial_.alloc(kReduceScratch);
+    SFEM_CUDA(cudaMemset(partial_.p, 0, sizeof(double) * kReduceScratch));
     scal_.alloc(1);
     step_.alloc(2);
     // smoother spectra
     for (size_t l = 1; l < levels_.size(); ++l) estimate_eigenvalues(levels_[l]);
     build_coarse();
-    d_in_.alloc(fine.m);
-    d_out_.alloc(fine.m);
     SFEM_CUDA(cudaDeviceSynchronize());
   }
 
@@ -684,9 +727,127 @@ class MultigridImpl final : public Multigrid {
   }
   bool learned_active() const override { return use_learned_; }
 
+  void dot_to(const T* x, const T* y, int64_t n, double* out, cudaStream_t s) {
+    launch_pdl(vec_dot<T>, kReduceBlocks, kReduceThreads, 0, s, n, x, y, partial_.p, out);
+  }
+  static constexpr int block_slots(int p) { return ((4 * p + 1) * (4 * p + 1) * (4 * p + 1) + 63) / 64 * 64; }
+  template <int PF>
+  static size_t prolongate_smem() {
+    return 64 + sizeof(T) * block_slots(PF - 1) + 2 * 6 * size_t(block_slots(PF));
+  }
+  template <int PF>
+  static size_t restrict_smem(size_t n_list) {
+    return 64 + sizeof(T) * block_slots(PF) + 2 * n_list;
+  }
+
+  // Tables of the p-transfer by blocks, from the embedding matrix of one cell: the
+  // first cell of a full block that holds a fine node gives its coarse nodes and
+  // weights (any cell would: the coarse function is continuous).
+  void build_block_transfer(Level& F, const Level& C) {
+    const BlockView* vf = F.op->block_view();
+    const BlockView* vc = C.op->block_view();
+    // (fewer blocks than SMs: the thread-per-cell forms are as fast)
+    if (!vf || !vc || vf->n_blocks != vc->n_blocks || vf->n_blocks < 148) return;
+    const int pf = F.degree, pc = C.degree;
+    const int NF1 = 4 * pf + 1, NC1 = 4 * pc + 1, NBF = block_slots(pf), NBC = block_slots(pc);
+    const KuhnOffsets of(pf), oc(pc);
+    std::vector<int> cslot(NC1 * NC1 * NC1), fslot(NF1 * NF1 * NF1);
+    for (size_t n = 0; n < vc->lattice.size(); ++n) cslot[vc->lattice[n]] = int(n);
+    for (size_t n = 0; n < vf->lattice.size(); ++n) fslot[vf->lattice[n]] = int(n);
+    std::vector<double> w;  // distinct weights
+    auto weight = [&](double v) {
+      for (size_t k = 0; k < w.size(); ++k)
+        if (w[k] == v) return int(k);
+      w.push_back(v);
+      return int(w.size()) - 1;
+    };
+    std::vector<uint16_t> ent(6 * size_t(NBF), uint16_t(7 << 12));
+    std::vector<uint8_t> hi(NBF, 0);
+    std::vector<char> seen(NBF, 0);
+    std::vector<std::vector<uint16_t>> lists(NBC);
+    for (int h = 0; h < 64; ++h)
+      for (int q = 0; q < 6; ++q)
+        for (int i = 0; i < F.Kf; ++i) {
+          const int hx = h & 3, hy = (h >> 2) & 3, hz = h >> 4;
+          const int x = pf * hx + of.off[q][i][0], y = pf * hy + of.off[q][i][1], z = pf * hz + of.off[q][i][2];
+          const int n = fslot[x + NF1 * (y + NF1 * z)];
+          if (seen[n]) continue;
+          seen[n] = 1;
+          hi[n] = uint8_t((x == 4 * pf) | (y == 4 * pf) << 1 | (z == 4 * pf) << 2);
+          int e = 0;
+          for (int j = 0; j < F.Kc; ++j) {
+            const double v = F.mats_host[size_t(i) * F.Kc + j];
+            if (v == 0.0) continue;
+            const int s = cslot[pc * hx + oc.off[q][j][0] + NC1 * (pc * hy + oc.off[q][j][1] + NC1 * (pc * hz + oc.off[q][j][2]))];
+            const int k = weight(v);
+            SFEM_REQUIRE(e < 6 && k < 7, FEM_ERR_INTERNAL, "block transfer: unexpected embedding");
+            ent[size_t(e++) * NBF + n] = uint16_t(s | k << 12);
+            lists[s].push_back(uint16_t(n | k << 12));
+          }
+        }
+    std::vector<uint16_t> list, order(NBC);
+    std::vector<int32_t> start(NBC + 1, 0);
+    for (int s = 0; s < NBC; ++s) {
+      list.insert(list.end(), lists[s].begin(), lists[s].end());
+      start[s + 1] = int32_t(list.size());
+      order[s] = uint16_t(s);
+    }
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return lists[a].size() > lists[b].size(); });
+    for (size_t k = 0; k < w.size(); ++k) F.bt_w.w[k] = w[k];
+    F.bt_ent.upload(ent);
+    F.bt_hi.upload(hi);
+    F.bt_list.upload(list);
+    F.bt_start.upload(start);
+    F.bt_order.upload(order);
+    int dev = 0, sms = 0;
+    SFEM_CUDA(cudaGetDevice(&dev));
+    SFEM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    auto fit = [&](auto kernel, size_t smem) {
+      int occ = 0;
+      SFEM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+      SFEM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kXferThreads, smem));
+      return int(std::min<int64_t>(vf->n_blocks, int64_t(occ) * sms));
+    };
+    auto setup = [&](auto pt) {
+      constexpr int PF = decltype(pt)::value, NF = block_slots(PF), NC = block_slots(PF - 1);
+      F.bt_grid[0] = fit(block_prolongate_add<T, NF, NC>, prolongate_smem<PF>());
+      F.bt_grid[1] = std::min(fit(block_restrict_add<T, NF, NC, false>, restrict_smem<PF>(list.size())),
+                              fit(block_restrict_add<T, NF, NC, true>, restrict_smem<PF>(list.size())));
+    };
+    if (pf == 2) setup(std::integral_constant<int, 2>{});
+    else setup(std::integral_constant<int, 3>{});
+    F.by_blocks = F.bt_grid[0] > 0 && F.bt_grid[1] > 0;
+  }
+
+  BlockTransferTables block_tables(const Level& F) const {
+    return {F.bt_ent.p, F.bt_hi.p, F.bt_list.p, F.bt_start.p, F.bt_order.p, int32_t(F.bt_list.n)};
+  }
+  void prolongate_blocks(const Level& F, const Level& C, const T* xc, T* xf, cudaStream_t s) {
+    const BlockView &vf = *F.op->block_view(), &vc = *C.op->block_view();
+    if (F.degree == 2)
+      launch_pdl(block_prolongate_add<T, block_slots(2), block_slots(1)>, F.bt_grid[0], kXferThreads, prolongate_smem<2>(),
+                 s, vf.n_blocks, block_tables(F), F.bt_w, vf.upper, vf.codes, vc.codes, xc, xf);
+    else
+      launch_pdl(block_prolongate_add<T, block_slots(3), block_slots(2)>, F.bt_grid[0], kXferThreads, prolongate_smem<3>(),
+                 s, vf.n_blocks, block_tables(F), F.bt_w, vf.upper, vf.codes, vc.codes, xc, xf);
+  }
+  // xc += P^T (xf - tf), tf may be null
+  void restrict_blocks(const Level& F, const Level& C, const T* xf, const T* tf, T* xc, cudaStream_t s) {
+    const BlockView &vf = *F.op->block_view(), &vc = *C.op->block_view();
+    auto go = [&](auto pt, auto mt) {
+      constexpr int PF = decltype(pt)::value;
+      launch_pdl(block_restrict_add<T, block_slots(PF), block_slots(PF - 1), decltype(mt)::value>, F.bt_grid[1],
+                 kXferThreads, restrict_smem<PF>(F.bt_list.n), s, vf.n_blocks, block_tables(F), F.bt_w, vf.upper,
+                 vf.codes, vc.codes, xf, tf, xc);
+    };
+    using P2 = std::integral_constant<int, 2>;
+    using P3 = std::integral_constant<int, 3>;
+    if (F.degree == 2) tf ? go(P2{}, std::true_type{}) : go(P2{}, std::false_type{});
+    else tf ? go(P3{}, std::true_type{}) : go(P3{}, std::false_type{});
+  }
+
   double dot(const T* x, const T* y, int64_t n, cudaStream_t s) {
-    vec_dot_partial<T><<<kReduceBlocks, kReduceThreads, 0, s>>>(n, x, y, partial_.p);
-    reduce_partials<<<1, kReduceThreads, 0, s>>>(kReduceBlocks, partial_.p, scal_.p);
+    dot_to(x, y, n, scal_.p, s);
     double h = 0;
     SFEM_CUDA(cudaMemcpyAsync(&h, scal_.p, sizeof(double), cudaMemcpyDeviceToHost, s));
     SFEM_CUDA(cudaStreamSynchronize(s));
@@ -727,6 +888,7 @@ class MultigridImpl final : public Multigrid {
       vec_axpby<T><<<g, 256, 0, s>>>(m, T(1), L.d.p, T(bt), L.x.p);       // p = z + b p
       rz = rz_new;
     }
+    clear_t(L, s);
     const int k = int(alpha.size());
     SFEM_REQUIRE(k > 0, FEM_ERR_INTERNAL, "multigrid: eigenvalue estimate failed");
     std::vector<double> da(k), ob(k > 1 ? k - 1 : 0);
@@ -810,19 +972,45 @@ class MultigridImpl final : public Multigrid {
     const double theta = 0.5 * (L.lmax + L.lmin), delta = 0.5 * (L.lmax - L.lmin);
     double rho = delta / theta;
     if (zero_init) {
-      cheb_first_zero<T><<<g, 256, 0, s>>>(m, T(1.0 / theta), L.inv_diag.p, b, L.d.p, x);
+      launch_pdl(cheb_first_zero<T>, g, 256, 0, s, m, T(1.0 / theta), L.inv_diag.p, b, L.d.p, x);
     } else {
-      L.op->vmult(L.t.p, x, s);
-      cheb_step<T, true><<<g, 256, 0, s>>>(m, T(0), T(1.0 / theta), L.inv_diag.p, b, L.t.p, L.d.p, x);
+      product(L, x, s);
+      cheb<true>(L, T(0), T(1.0 / theta), b, x, s);
     }
     for (int k = 1; k < params.smoother_degree; ++k) {
       const double rho_new = 1.0 / (2.0 * theta / delta - rho);
-      L.op->vmult(L.t.p, x, s);
-      cheb_step<T><<<g, 256, 0, s>>>(m, T(rho_new * rho), T(2.0 * rho_new / delta), L.inv_diag.p, b, L.t.p,
-                                     L.d.p, x);
+      product(L, x, s);
+      cheb<false>(L, T(rho_new * rho), T(2.0 * rho_new / delta), b, x, s);
       rho = rho_new;
     }
     SFEM_CUDA(cudaGetLastError());
+  }
+
+  // t = A x.  On levels with clear_t operators that add into their result find t
+  // zero: every reader of t (cheb, residual) clears it, so that no product needs a
+  // fill of its own.
+  void product(Level& L, const T* x, cudaStream_t s) {
+    if (L.clear_t) L.op->vmult_zeroed(L.t.p, x, s);
+    else L.op->vmult(L.t.p, x, s);
+  }
+  template <bool FIRST>
+  void cheb(Level& L, T f1, T f2, const T* b, T* x, cudaStream_t s) {
+    const int64_t m = L.op->m;
+    if (L.clear_t)
+      launch_pdl(cheb_step<T, FIRST, true>, grid_for(m), 256, 0, s, m, f1, f2, L.inv_diag.p, b, L.t.p, L.d.p, x, 0);
+    else
+      launch_pdl(cheb_step<T, FIRST, false>, grid_for(m), 256, 0, s, m, f1, f2, L.inv_diag.p, b, L.t.p, L.d.p, x, 0);
+  }
+  // r = b - t, and z = 0 (z may be null)
+  void residual(Level& L, const T* b, T* r, T* z, int64_t nz, cudaStream_t s) {
+    const int64_t m = L.op->m;
+    if (L.clear_t)
+      launch_pdl(vec_residual<T, true>, grid_for(m), 256, 0, s, m, b, L.t.p, r, z, nz, 0);
+    else
+      launch_pdl(vec_residual<T, false>, grid_for(m), 256, 0, s, m, b, L.t.p, r, z, nz, 0);
+  }
+  void clear_t(Level& L, cudaStream_t s) {
+    if (L.clear_t) SFEM_CUDA(cudaMemsetAsync(L.t.p, 0, sizeof(T) * L.op->m, s));
   }
 
   template <int KF, int KC>
@@ -839,20 +1027,24 @@ class MultigridImpl final : public Multigrid {
     const Level& Cl = levels_[l - 1];
     const unsigned grid = unsigned((F.op->n_cells + 127) / 128);
     if (F.ttype == Level::T_DGP) {
-      dg_p_prolongate_add<T><<<grid, 128, 0, s>>>(F.op->n_cells, F.Kf, F.Kc, F.mats.p, static_cast<const T*>(src),
+      launch_pdl(dg_p_prolongate_add<T>, grid, 128, 0, s, F.op->n_cells, F.Kf, F.Kc, F.mats.p, static_cast<const T*>(src),
                                                   static_cast<T*>(dst));
       SFEM_CUDA(cudaGetLastError());
       return;
     }
     if (F.ttype == Level::T_C) {
-      c_prolongate_add<T><<<grid, 128, 0, s>>>(F.op->n_cells, F.Kf, Cl.op->device_dof_table(),
+      launch_pdl(c_prolongate_add<T>, grid, 128, 0, s, F.op->n_cells, F.Kf, Cl.op->device_dof_table(),
                                                static_cast<const T*>(src), static_cast<T*>(dst));
       SFEM_CUDA(cudaGetLastError());
       return;
     }
+    if (F.by_blocks) {
+      prolongate_blocks(F, Cl, static_cast<const T*>(src), static_cast<T*>(dst), s);
+      return;
+    }
 #define SFEM_PXFER(KF_, KC_)                                                                               \
   if (F.Kf == KF_ && F.Kc == KC_) {                                                                        \
-    transfer_p_prolongate_k<T, KF_, KC_><<<grid, 128, 0, s>>>(                                             \
+    launch_pdl(transfer_p_prolongate_k<T, KF_, KC_>, grid, 128, 0, s,                                              \
         F.op->n_cells, F.owner.p, xfer_mat<KF_, KC_>(F), F.op->device_dof_table(), Cl.op->device_dof_table(), \
         static_cast<const T*>(src), static_cast<T*>(dst));                                                 \
     SFEM_CUDA(cudaGetLastError());                                                                        \
@@ -864,7 +1056,7 @@ class MultigridImpl final : public Multigrid {
 #undef SFEM_PXFER
 #define SFEM_XFER(KF_, KC_)                                                                                \
   if (F.Kf == KF_ && F.Kc == KC_) {                                                                        \
-    transfer_prolongate_add_k<T, KF_, KC_><<<grid, 128, 0, s>>>(                                           \
+    launch_pdl(transfer_prolongate_add_k<T, KF_, KC_>, grid, 128, 0, s,                                            \
         F.op->n_cells, F.parent.p, F.mat_id.p, F.owner.p, F.mats.p, F.op->device_dof_table(),               \
         Cl.op->device_dof_table(), Cl.op->n_cells, static_cast<const T*>(src), static_cast<T*>(dst));       \
     SFEM_CUDA(cudaGetLastError());                                                                        \
@@ -872,7 +1064,7 @@ class MultigridImpl final : public Multigrid {
   }
     SFEM_XFER(20, 10) SFEM_XFER(10, 4) SFEM_XFER(4, 4) SFEM_XFER(10, 10) SFEM_XFER(20, 20)
 #undef SFEM_XFER
-    transfer_prolongate_add<T><<<grid, 128, 0, s>>>(
+    launch_pdl(transfer_prolongate_add<T>, grid, 128, 0, s, 
         F.op->n_cells, F.Kf, F.Kc, F.parent.p, F.mat_id.p, F.owner.p, F.mats.p, F.op->device_dof_table(),
         Cl.op->device_dof_table(), Cl.op->n_cells, static_cast<const T*>(src), static_cast<T*>(dst));
     SFEM_CUDA(cudaGetLastError());
@@ -884,20 +1076,24 @@ class MultigridImpl final : public Multigrid {
     const Level& Cl = levels_[l - 1];
     const unsigned grid = unsigned((F.op->n_cells + 127) / 128);
     if (F.ttype == Level::T_DGP) {
-      dg_p_restrict_add<T><<<grid, 128, 0, s>>>(F.op->n_cells, F.Kf, F.Kc, F.mats.p, static_cast<const T*>(src),
+      launch_pdl(dg_p_restrict_add<T>, grid, 128, 0, s, F.op->n_cells, F.Kf, F.Kc, F.mats.p, static_cast<const T*>(src),
                                                 static_cast<T*>(dst));
       SFEM_CUDA(cudaGetLastError());
       return;
     }
     if (F.ttype == Level::T_C) {
-      c_restrict_add<T><<<grid, 128, 0, s>>>(F.op->n_cells, F.Kf, Cl.op->device_dof_table(),
+      launch_pdl(c_restrict_add<T>, grid, 128, 0, s, F.op->n_cells, F.Kf, Cl.op->device_dof_table(),
                                              static_cast<const T*>(src), static_cast<T*>(dst));
       SFEM_CUDA(cudaGetLastError());
       return;
     }
+    if (F.by_blocks) {
+      restrict_blocks(F, Cl, static_cast<const T*>(src), nullptr, static_cast<T*>(dst), s);
+      return;
+    }
 #define SFEM_PXFER(KF_, KC_)                                                                               \
   if (F.Kf == KF_ && F.Kc == KC_) {                                                                        \
-    transfer_p_restrict_k<T, KF_, KC_><<<grid, 128, 0, s>>>(                                               \
+    launch_pdl(transfer_p_restrict_k<T, KF_, KC_>, grid, 128, 0, s,                                                \
         F.op->n_cells, F.owner.p, xfer_mat<KF_, KC_>(F), F.op->device_dof_table(), Cl.op->device_dof_table(), \
         static_cast<const T*>(src), static_cast<T*>(dst));                                                 \
     SFEM_CUDA(cudaGetLastError());                                                                        \
@@ -909,7 +1105,7 @@ class MultigridImpl final : public Multigrid {
 #undef SFEM_PXFER
 #define SFEM_XFER(KF_, KC_)                                                                                \
   if (F.Kf == KF_ && F.Kc == KC_) {                                                                        \
-    transfer_restrict_add_k<T, KF_, KC_><<<grid, 128, 0, s>>>(                                             \
+    launch_pdl(transfer_restrict_add_k<T, KF_, KC_>, grid, 128, 0, s,                                              \
         F.op->n_cells, F.parent.p, F.mat_id.p, F.owner.p, F.mats.p, F.op->device_dof_table(),               \
         Cl.op->device_dof_table(), Cl.op->n_cells, static_cast<const T*>(src), static_cast<T*>(dst));       \
     SFEM_CUDA(cudaGetLastError());                                                                        \
@@ -917,14 +1113,14 @@ class MultigridImpl final : public Multigrid {
   }
     SFEM_XFER(20, 10) SFEM_XFER(10, 4) SFEM_XFER(4, 4) SFEM_XFER(10, 10) SFEM_XFER(20, 20)
 #undef SFEM_XFER
-    transfer_restrict_add<T><<<grid, 128, 0, s>>>(
+    launch_pdl(transfer_restrict_add<T>, grid, 128, 0, s, 
         F.op->n_cells, F.Kf, F.Kc, F.parent.p, F.mat_id.p, F.owner.p, F.mats.p, F.op->device_dof_table(),
         Cl.op->device_dof_table(), Cl.op->n_cells, static_cast<const T*>(src), static_cast<T*>(dst));
     SFEM_CUDA(cudaGetLastError());
   }
 
   void coarse_solve(void* dst, const void* src, cudaStream_t s) override {
-    dense_matvec<T><<<unsigned((coarse_n_ * 32 + 255) / 256), 256, 0, s>>>(
+    launch_pdl(dense_matvec<T>, unsigned((coarse_n_ * 32 + 255) / 256), 256, 0, s, 
         coarse_n_, coarse_inv_.p, static_cast<const T*>(src), static_cast<T*>(dst));
     SFEM_CUDA(cudaGetLastError());
   }
@@ -939,31 +1135,41 @@ class MultigridImpl final : public Multigrid {
     const int64_t m = L.op->m;
     const unsigned g = grid_for(m);
     const bool learned = use_learned_ && l == int(levels_.size()) - 1;
+    Level& C = levels_[l - 1];
+    bool restricted = false;
     if (learned) {
       SFEM_CUDA(cudaMemsetAsync(L.x.p, 0, sizeof(T) * m, s));
       if (params.learned_steps & 1) {
         // pre-smoothing from zero: x = w z, z = S(b), w = (b,z)/(z,Az); r = b - w Az
         learned_step(L, L.b.p, s);
-        residual_ratio<T><<<g, 256, 0, s>>>(m, step_.p, L.b.p, L.t.p, L.r.p);
+        launch_pdl(residual_ratio<T>, g, 256, 0, s, m, step_.p, L.b.p, L.t.p, L.r.p);
+        clear_t(L, s);
       } else {
         SFEM_CUDA(cudaMemcpyAsync(L.r.p, L.b.p, sizeof(T) * m, cudaMemcpyDeviceToDevice, s));
       }
+      SFEM_CUDA(cudaMemsetAsync(C.b.p, 0, sizeof(T) * C.op->m, s));
     } else {
       smooth(l, L.x.p, L.b.p, true, s);
-      L.op->vmult(L.t.p, L.x.p, s);
-      vec_residual<T><<<g, 256, 0, s>>>(m, L.b.p, L.t.p, L.r.p);
+      product(L, L.x.p, s);
+      if (L.by_blocks && !L.clear_t) {
+        // the restriction forms the residual itself
+        SFEM_CUDA(cudaMemsetAsync(C.b.p, 0, sizeof(T) * C.op->m, s));
+        restrict_blocks(L, C, L.b.p, L.t.p, C.b.p, s);
+        restricted = true;
+      } else {
+        residual(L, L.b.p, L.r.p, C.b.p, C.op->m, s);
+      }
     }
-    Level& C = levels_[l - 1];
-    SFEM_CUDA(cudaMemsetAsync(C.b.p, 0, sizeof(T) * C.op->m, s));
-    restrict_add(l, C.b.p, L.r.p, s);
+    if (!restricted) restrict_add(l, C.b.p, L.r.p, s);
     cycle(l - 1, s);
     prolongate_add(l, L.x.p, C.x.p, s);
     if (learned) {
       if (!(params.learned_steps & 2)) return;
       // post-smoothing: one energy-optimal step along S(b - A x)
-      L.op->vmult(L.t.p, L.x.p, s);
-      vec_residual<T><<<g, 256, 0, s>>>(m, L.b.p, L.t.p, L.r.p);
+      product(L, L.x.p, s);
+      residual(L, L.b.p, L.r.p, nullptr, 0, s);
       learned_step(L, L.r.p, s);
+      clear_t(L, s);
     } else {
       smooth(l, L.x.p, L.b.p, false, s);
     }
@@ -972,17 +1178,16 @@ class MultigridImpl final : public Multigrid {
   // Learned smoothing step for residual r: z = S(r) (into L.d), A z (into L.t),
   // x += w z with the energy-optimal w = (r,z)/(z,Az); step_ keeps (r,z),(z,Az)
   // on the device so the step needs no host synchronisation (graph capturable).
-  // Any direction z with (r,z) > 0 then lowers the A-norm of the error.
+  // Any direction z with (r,z) > 0 then lowers the A-norm of the error.  t holds
+  // A z afterwards: the caller clears it when it is done with it.
   void learned_step(Level& L, const T* r, cudaStream_t s) {
     const int64_t m = L.op->m;
     SFEM_CUDA(cudaMemsetAsync(L.d.p, 0, sizeof(T) * m, s));
     learned_->apply(*L.op, r, L.d.p, s);
-    L.op->vmult(L.t.p, L.d.p, s);
-    vec_dot_partial<T><<<kReduceBlocks, kReduceThreads, 0, s>>>(m, r, L.d.p, partial_.p);
-    reduce_partials<<<1, kReduceThreads, 0, s>>>(kReduceBlocks, partial_.p, step_.p);
-    vec_dot_partial<T><<<kReduceBlocks, kReduceThreads, 0, s>>>(m, L.d.p, L.t.p, partial_.p);
-    reduce_partials<<<1, kReduceThreads, 0, s>>>(kReduceBlocks, partial_.p, step_.p + 1);
-    axpy_ratio<T><<<grid_for(m), 256, 0, s>>>(m, step_.p, L.d.p, L.x.p);
+    product(L, L.d.p, s);
+    dot_to(r, L.d.p, m, step_.p, s);
+    dot_to(L.d.p, L.t.p, m, step_.p + 1, s);
+    launch_pdl(axpy_ratio<T>, grid_for(m), 256, 0, s, m, step_.p, L.d.p, L.x.p);
     SFEM_CUDA(cudaGetLastError());
   }
 
@@ -1005,8 +1210,8 @@ class MultigridImpl final : public Multigrid {
     SFEM_CUDA(cudaMemsetAsync(cc_y_.p, 0, sizeof(T) * mc, s));
     // y += V(R r - A_c y): V-cycle iteration on the level below
     for (int it = 0; it < iterations; ++it) {
-      C.op->vmult(C.t.p, cc_y_.p, s);
-      vec_residual<T><<<grid_for(mc), 256, 0, s>>>(mc, cc_rhs_.p, C.t.p, C.b.p);
+      product(C, cc_y_.p, s);
+      residual(C, cc_rhs_.p, C.b.p, nullptr, 0, s);
       cycle(top - 1, s);
       vec_axpby<T><<<grid_for(mc), 256, 0, s>>>(mc, T(1), C.x.p, T(1), cc_y_.p);
     }
@@ -1016,34 +1221,31 @@ class MultigridImpl final : public Multigrid {
     SFEM_CUDA(cudaGetLastError());
   }
 
-  void run_cycle(cudaStream_t s) {
-    Level& top = levels_.back();
-    const int64_t m = top.op->m;
-    vec_convert<T, double><<<grid_for(m), 256, 0, s>>>(m, d_in_.p, top.b.p);
-    cycle(int(levels_.size()) - 1, s);
-    vec_convert<double, T><<<grid_for(m), 256, 0, s>>>(m, top.x.p, d_out_.p);
-    SFEM_CUDA(cudaGetLastError());
-  }
-
+  // dst = V(src).  The graph holds the cycle on the hierarchy's own vectors; the
+  // conversions to and from the caller's are launched around it, so that the
+  // vectors are not copied in between.
   void vcycle(double* dst, const double* src, cudaStream_t s) override {
-    SFEM_CUDA(cudaMemcpyAsync(d_in_.p, src, sizeof(double) * fine_m_, cudaMemcpyDeviceToDevice, s));
+    Level& top = levels_.back();
+    const int l = int(levels_.size()) - 1;
+    const int64_t m = top.op->m;
+    launch_pdl(vec_convert<T, double>, grid_for(m), 256, 0, s, m, src, top.b.p);
     if (params.use_graph) {
       const int mode = use_learned_ ? 1 : 0;
       if (!exec_[mode]) {
         // one eager cycle sets up kernel attributes and bindings, then capture
-        run_cycle(s);
+        cycle(l, s);
         SFEM_CUDA(cudaStreamSynchronize(s));
         if (!cap_stream_) SFEM_CUDA(cudaStreamCreateWithFlags(&cap_stream_, cudaStreamNonBlocking));
         SFEM_CUDA(cudaStreamBeginCapture(cap_stream_, cudaStreamCaptureModeThreadLocal));
-        run_cycle(cap_stream_);
+        cycle(l, cap_stream_);
         SFEM_CUDA(cudaStreamEndCapture(cap_stream_, &graph_[mode]));
         SFEM_CUDA(cudaGraphInstantiate(&exec_[mode], graph_[mode], 0));
       }
       SFEM_CUDA(cudaGraphLaunch(exec_[mode], s));
     } else {
-      run_cycle(s);
+      cycle(l, s);
     }
-    SFEM_CUDA(cudaMemcpyAsync(dst, d_out_.p, sizeof(double) * fine_m_, cudaMemcpyDeviceToDevice, s));
+    launch_pdl(vec_convert<double, T>, grid_for(m), 256, 0, s, m, top.x.p, dst);
   }
 };
 
@@ -1064,7 +1266,8 @@ CGSolver::CGSolver(Operator& A, Preconditioner* M, bool flexible) : A_(A), M_(M)
   p_.alloc(m);
   q_.alloc(m);
   if (flexible) zold_.alloc(m);
-  partial_.alloc(kReduceBlocks + 1);
+  partial_.alloc(kReduceScratch);
+  SFEM_CUDA(cudaMemset(partial_.p, 0, sizeof(double) * kReduceScratch));
   sc_.alloc(8);
   SFEM_CUDA(cudaMallocHost(&host_, 2 * sizeof(double)));
 }
@@ -1074,14 +1277,13 @@ CGSolver::~CGSolver() {
 }
 
 void CGSolver::dot_to(const double* x, const double* y, int slot, cudaStream_t s) {
-  vec_dot_partial<double><<<kReduceBlocks, kReduceThreads, 0, s>>>(A_.m, x, y, partial_.p);
-  reduce_partials<<<1, kReduceThreads, 0, s>>>(kReduceBlocks, partial_.p, sc_.p + slot);
+  launch_pdl(vec_dot<double>, kReduceBlocks, kReduceThreads, 0, s, A_.m, x, y, partial_.p, sc_.p + slot);
 }
 
 double CGSolver::dot(const double* x, const double* y, cudaStream_t s) {
-  vec_dot_partial<double><<<kReduceBlocks, kReduceThreads, 0, s>>>(A_.m, x, y, partial_.p);
-  reduce_partials<<<1, kReduceThreads, 0, s>>>(kReduceBlocks, partial_.p, partial_.p + kReduceBlocks);
-  SFEM_CUDA(cudaMemcpyAsync(host_, partial_.p + kReduceBlocks, sizeof(double), cudaMemcpyDeviceToHost, s));
+  constexpr int kScratch = 7;
+  dot_to(x, y, kScratch, s);
+  SFEM_CUDA(cudaMemcpyAsync(host_, sc_.p + kScratch, sizeof(double), cudaMemcpyDeviceToHost, s));
   SFEM_CUDA(cudaStreamSynchronize(s));
   return *host_;
 }
@@ -1092,8 +1294,11 @@ SolveInfo CGSolver::solve(double* x, const double* b, double rtol, int maxit, cu
   const unsigned g = grid_for(m);
   if (M_) M_->on_solve_start();
   // r = b - A x
+  // (q is zero between products where clear_in_passing says so)
+  const bool clear_q = clear_in_passing(A_);
   A_.vmult(q_.p, x, s);
-  vec_residual<double><<<g, 256, 0, s>>>(m, b, q_.p, r_.p);
+  if (clear_q) launch_pdl(vec_residual<double, true>, g, 256, 0, s, m, b, q_.p, r_.p, nullptr, 0, 0);
+  else launch_pdl(vec_residual<double, false>, g, 256, 0, s, m, b, q_.p, r_.p, nullptr, 0, 0);
   const double bnorm = std::sqrt(dot(b, b, s));
   double rr = dot(r_.p, r_.p, s);
   info.r0 = std::sqrt(rr);
@@ -1118,10 +1323,15 @@ SolveInfo CGSolver::solve(double* x, const double* b, double rtol, int maxit, cu
   double prev_rn = info.r0;
   info.status = FEM_ERR_NOT_CONVERGED;
   for (int it = 1; it <= maxit; ++it) {
-    A_.vmult(q_.p, p_.p, s);
+    if (clear_q) A_.vmult_zeroed(q_.p, p_.p, s);
+    else A_.vmult(q_.p, p_.p, s);
     dot_to(p_.p, q_.p, kPQ, s);
-    cg_update_xr_dev<<<g, 256, 0, s>>>(m, sc_.p, cur, kPQ, p_.p, q_.p, x, r_.p);
-    dot_to(r_.p, r_.p, kRR, s);
+    if (clear_q)
+      launch_pdl(cg_update_xr<true>, kReduceBlocks, kReduceThreads, 0, s, m, sc_.p, cur, kPQ, kRR, p_.p, q_.p, x, r_.p,
+                 partial_.p, 0);
+    else
+      launch_pdl(cg_update_xr<false>, kReduceBlocks, kReduceThreads, 0, s, m, sc_.p, cur, kPQ, kRR, p_.p, q_.p, x,
+                 r_.p, partial_.p, 0);
     SFEM_CUDA(cudaMemcpyAsync(host_, sc_.p + kPQ, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
     SFEM_CUDA(cudaStreamSynchronize(s));
     const double pq = host_[0];
@@ -1155,7 +1365,7 @@ SolveInfo CGSolver::solve(double* x, const double* b, double rtol, int maxit, cu
     dot_to(r_.p, z_.p, 1 - cur, s);
     if (flexible_) dot_to(r_.p, zold_.p, kRZOLD, s);
     // p = z + beta p, beta = (r,z)_new / (r,z), or ((r,z)_new - (r,z_old)) / (r,z)
-    cg_update_p_dev<<<g, 256, 0, s>>>(m, 1.0, sc_.p, 1 - cur, flexible_ ? kRZOLD : -1, cur, z_.p, p_.p);
+    launch_pdl(cg_update_p_dev, g, 256, 0, s, m, 1.0, sc_.p, 1 - cur, flexible_ ? kRZOLD : -1, cur, z_.p, p_.p);
     cur = 1 - cur;
   }
   SFEM_CUDA(cudaGetLastError());
@@ -1169,8 +1379,7 @@ JacobiPreconditioner::JacobiPreconditioner(Operator& A) {
 }
 
 void JacobiPreconditioner::apply(double* dst, const double* src, cudaStream_t s) {
-  vec_scale<double><<<grid_for(int64_t(inv_.n)), 256, 0, s>>>(int64_t(inv_.n), inv_.p, src, dst);
-  SFEM_CUDA(cudaGetLastError());
+  launch_pdl(vec_scale<double>, grid_for(int64_t(inv_.n)), 256, 0, s, int64_t(inv_.n), inv_.p, src, dst);
 }
 
 }  // namespace sfem

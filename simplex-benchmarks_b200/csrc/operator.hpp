@@ -65,6 +65,14 @@ struct OpConfig {
   bool weak_bc = false;    // CG: weak (Nitsche) Dirichlet on the boundary faces, no constrained DoFs
 };
 
+// Blocks of 4 x 4 x 4 hexes of a CG operator on a Kuhn box (kernels_cg_block.cuh)
+struct BlockView {
+  int64_t n_blocks = 0;
+  const int32_t* codes = nullptr;   // device [n_blocks][NBP]
+  const uint8_t* upper = nullptr;   // device [n_blocks]
+  std::vector<int32_t> lattice;     // lattice node of every slot
+};
+
 struct HostPipe;  // staging buffers and streams of vmult_host (host_vmult.cu)
 
 class Operator {
@@ -84,11 +92,17 @@ class Operator {
 
   size_t elem_size() const { return cfg.precision == FEM_FP64 ? 8 : 4; }
   virtual void vmult(void* dst, const void* src, cudaStream_t s) = 0;
+  // vmult onto a dst that is zero already where needs_zero() (callers that zero
+  // it in passing save the fill)
+  virtual bool needs_zero() const { return false; }
+  virtual void vmult_zeroed(void* dst, const void* src, cudaStream_t s) { vmult(dst, src, s); }
   // phase 1 / phase 2 of vmult (see fem_op_vmult_phase)
   virtual void vmult_phase(void* dst, const void* src, int phase, cudaStream_t s) = 0;
   virtual void diagonal(void* diag, cudaStream_t s) = 0;
   // CG: device table [K][n_cells] of global DoFs, -1 at constrained ones
   virtual const int32_t* device_dof_table() const { return nullptr; }
+  // CG on a Kuhn box: its blocks (nullptr: none)
+  virtual const BlockView* block_view() const { return nullptr; }
   // Device scratch one vmult needs (DG: the published face traces; CG: none).
   virtual size_t scratch_bytes() const { return 0; }
   // vmult with the scratch supplied by the caller instead of the operator's own.

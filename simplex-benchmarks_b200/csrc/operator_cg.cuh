@@ -368,9 +368,9 @@ class CGOperator final : public Operator {
   }
   template <int P, int NB, int KP>
   void launch_cube(const T* x, T* d, int sched, cudaStream_t s) {
-    cg_cube_pipe_kernel<P, T, NB, KP><<<unsigned(cube_grid), 384, cube_smem<P, NB, KP>(), s>>>(
-        n_blocks, d_tmapv.p, d_bdof.p, d_ritem[sched].p, d_cslot8[sched].p, d_geo.p, x, d, d_constrained.n,
-        d_constrained.p);
+    launch_pdl(cg_cube_pipe_kernel<P, T, NB, KP>, unsigned(cube_grid), 384, cube_smem<P, NB, KP>(), s, n_blocks,
+               d_tmapv.p, d_bdof.p, d_ritem[sched].p, d_cslot8[sched].p, d_geo.p, x, d, int64_t(d_constrained.n),
+               d_constrained.p);
   }
 
   // TF32 tensor-core cube kernel (variant 8, FP32 operators with cube tables):
@@ -568,6 +568,8 @@ class CGOperator final : public Operator {
     vmult_phase(dst, src, 1, s);
     vmult_phase(dst, src, 2, s);
   }
+  bool needs_zero() const override { return true; }
+  void vmult_zeroed(void* dst, const void* src, cudaStream_t s) override { vmult_phase(dst, src, 2, s); }
 
   void vmult_phase(void* dst, const void* src, int phase, cudaStream_t s) override {
     T* d = static_cast<T*>(dst);
@@ -709,12 +711,12 @@ class CGOperator final : public Operator {
     const int64_t n = std::max<int64_t>(n_cells, int64_t(d_constrained.n));
     const unsigned grid = blocks_for(n, 128);
     switch (cfg.degree) {
-      case 1: cg_cell_kernel<1, T><<<grid, 128, 0, s>>>(n_cells, d_dofs.p, d_geo.p, x, d, d_constrained.n, d_constrained.p); break;
-      case 2: cg_cell_kernel<2, T><<<grid, 128, 0, s>>>(n_cells, d_dofs.p, d_geo.p, x, d, d_constrained.n, d_constrained.p); break;
+      case 1: launch_pdl(cg_cell_kernel<1, T>, grid, 128, 0, s, n_cells, d_dofs.p, d_geo.p, x, d, int64_t(d_constrained.n), d_constrained.p); break;
+      case 2: launch_pdl(cg_cell_kernel<2, T>, grid, 128, 0, s, n_cells, d_dofs.p, d_geo.p, x, d, int64_t(d_constrained.n), d_constrained.p); break;
       case 3:
         // P3 in FP64: registers capped for 4 CTAs per SM (measured faster on B200)
-        if (sizeof(T) == 8) cg_cell_kernel<3, T, 4><<<grid, 128, 0, s>>>(n_cells, d_dofs.p, d_geo.p, x, d, d_constrained.n, d_constrained.p);
-        else cg_cell_kernel<3, T><<<grid, 128, 0, s>>>(n_cells, d_dofs.p, d_geo.p, x, d, d_constrained.n, d_constrained.p);
+        if (sizeof(T) == 8) launch_pdl(cg_cell_kernel<3, T, 4>, grid, 128, 0, s, n_cells, d_dofs.p, d_geo.p, x, d, int64_t(d_constrained.n), d_constrained.p);
+        else launch_pdl(cg_cell_kernel<3, T>, grid, 128, 0, s, n_cells, d_dofs.p, d_geo.p, x, d, int64_t(d_constrained.n), d_constrained.p);
         break;
     }
     SFEM_CUDA(cudaGetLastError());
@@ -735,6 +737,7 @@ class CGOperator final : public Operator {
   }
 
   const int32_t* device_dof_table() const override { return d_dofs.p; }
+  const BlockView* block_view() const override { return blocks.view.n_blocks ? &blocks.view : nullptr; }
 
   void element_matrices(void* out, cudaStream_t s) override {
     T* m = static_cast<T*>(out);
@@ -834,9 +837,9 @@ class CGVectorOperator final : public Operator {
     }
     const unsigned grid = blocks_for(std::max<int64_t>(n_cells, int64_t(d_constrained.n)), 128);
     switch (cfg.degree) {
-      case 1: cg_cell_vec_kernel<1, T, NC><<<grid, 128, 0, s>>>(n_cells, d_dofs.p, d_geo.p, x, d, d_constrained.n, d_constrained.p); break;
-      case 2: cg_cell_vec_kernel<2, T, NC><<<grid, 128, 0, s>>>(n_cells, d_dofs.p, d_geo.p, x, d, d_constrained.n, d_constrained.p); break;
-      case 3: cg_cell_vec_kernel<3, T, NC><<<grid, 128, 0, s>>>(n_cells, d_dofs.p, d_geo.p, x, d, d_constrained.n, d_constrained.p); break;
+      case 1: launch_pdl(cg_cell_vec_kernel<1, T, NC>, grid, 128, 0, s, n_cells, d_dofs.p, d_geo.p, x, d, int64_t(d_constrained.n), d_constrained.p); break;
+      case 2: launch_pdl(cg_cell_vec_kernel<2, T, NC>, grid, 128, 0, s, n_cells, d_dofs.p, d_geo.p, x, d, int64_t(d_constrained.n), d_constrained.p); break;
+      case 3: launch_pdl(cg_cell_vec_kernel<3, T, NC>, grid, 128, 0, s, n_cells, d_dofs.p, d_geo.p, x, d, int64_t(d_constrained.n), d_constrained.p); break;
     }
     SFEM_CUDA(cudaGetLastError());
   }

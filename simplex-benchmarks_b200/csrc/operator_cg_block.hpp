@@ -21,6 +21,8 @@ constexpr int cg_block_min_ctas() {
 template <typename T, int NC>
 struct CGBlocks {
   DevBuf<int32_t> codes;
+  DevBuf<uint8_t> upper;
+  BlockView view;  // also without the kernel (P3 FP64): the multigrid's transfers go by blocks
   DevBuf<int16_t> pos;
   DevBuf<T> geo;
   int64_t n_blocks = 0;
@@ -29,10 +31,16 @@ struct CGBlocks {
   // geo_soa: metric values [6][n_cells] in the operator's precision
   void build(const Mesh& mesh, int p, const std::vector<int32_t>& cell_dofs, const std::vector<uint8_t>& constrained,
              const std::vector<T>& geo_soa) {
-    if (p == 3 && sizeof(T) == 8) return;  // the slower form there (see CGOperator::use_blocks)
     const std::vector<int32_t> lattice = p == 1 ? slots<1>() : p == 2 ? slots<2>() : slots<3>();
     const CGBlockTables tb = build_cg_block_tables(mesh, p, cell_dofs, constrained, lattice);
     if (!tb.n_blocks) return;
+    codes.upload(tb.codes);
+    upper.upload(tb.upper);
+    view.n_blocks = tb.n_blocks;
+    view.codes = codes.p;
+    view.upper = upper.p;
+    view.lattice = lattice;
+    if (p == 3 && sizeof(T) == 8) return;  // the slower kernel there (see CGOperator::use_blocks)
     std::vector<T> g(size_t(36) * 64 * tb.n_blocks);
 #pragma omp parallel for schedule(static)
     for (int64_t b = 0; b < tb.n_blocks; ++b)
@@ -43,7 +51,6 @@ struct CGBlocks {
             g[(36 * size_t(b) + 6 * q + k) * 64 + t] = c >= 0 ? geo_soa[size_t(k) * mesh.n_cells + c] : T(0);
         }
     geo.upload(g);
-    codes.upload(tb.codes);
     n_blocks = tb.n_blocks;
     switch (p) {
       case 1: setup<1>(lattice); break;
@@ -86,8 +93,8 @@ struct CGBlocks {
 
   template <int P>
   void launch(const T* x, T* d, int64_t n_constrained, const int32_t* constrained, cudaStream_t s) const {
-    kernel<P>()<<<unsigned(grid), 64, CGBlockShape<P, T>::bytes(NC), s>>>(n_blocks, codes.p, pos.p, geo.p, x, d,
-                                                                        n_constrained, constrained);
+    launch_pdl(kernel<P>(), unsigned(grid), 64, CGBlockShape<P, T>::bytes(NC), s, n_blocks, codes.p, pos.p, geo.p, x, d,
+               n_constrained, constrained);
   }
   void launch(int p, const T* x, T* d, int64_t n_constrained, const int32_t* constrained, cudaStream_t s) const {
     switch (p) {

@@ -317,7 +317,7 @@ class DGOperator final : public Operator {
       grid_per_dev[dev] = sms * occ;
     });
     const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(n_blocks, grid_per_dev[dev]));
-    kern<<<unsigned(grid), kQB, S::SMEM, s>>>(b, n_blocks, status);
+    launch_pdl(kern, unsigned(grid), kQB, S::SMEM, s, b, n_blocks, status);
   }
 
   // PDLM > 0 (scalar problems): the apply pass is launched as a programmatic
@@ -339,7 +339,7 @@ class DGOperator final : public Operator {
         int64_t nbt = 0;
         const DGBatch<T> bt = make_batch(probs, n, kQB, nbt);
         if (trace_tma_ok<P>(probs, n)) run_trace_tma<P>(bt, nbt, s, status);
-        else dg_trace_blk_kernel<P, T><<<unsigned(nbt), kQB, 0, s>>>(bt, nbt);
+        else launch_pdl(dg_trace_blk_kernel<P, T>, unsigned(nbt), kQB, 0, s, bt, nbt);
       } else {
         opt_in_smem(dg_trace_kernel<P, NC, BS, T>, sm_trace, conf_t);
         dg_trace_kernel<P, NC, BS, T><<<unsigned(n_blocks), BS, sm_trace, s>>>(b, n_blocks);
@@ -350,17 +350,7 @@ class DGOperator final : public Operator {
       // the trace pass just launched on this stream is the only producer the
       // apply pass may overlap: everything else it reads was complete before
       // the trace pass started
-      cudaLaunchConfig_t lc = {};
-      lc.gridDim = dim3(unsigned(n_blocks));
-      lc.blockDim = dim3(BS);
-      lc.dynamicSmemBytes = sm_apply;
-      lc.stream = s;
-      cudaLaunchAttribute at[1];
-      at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-      at[0].val.programmaticStreamSerializationAllowed = 1;
-      lc.attrs = at;
-      lc.numAttrs = 1;
-      SFEM_CUDA(cudaLaunchKernelEx(&lc, apply, b, n_blocks));
+      launch_pdl(apply, unsigned(n_blocks), BS, sm_apply, s, b, n_blocks);
     } else {
       apply<<<unsigned(n_blocks), BS, sm_apply, s>>>(b, n_blocks);
     }
@@ -379,7 +369,7 @@ class DGOperator final : public Operator {
     auto kern = dg_fused_kernel<P, NC, MASS, BS, T, dg_fused_min_ctas<P, NC, T>()>;
     // at most BS cells with four outer neighbours each
     opt_in_smem(kern, S::bytes(5 * BS), conf);
-    kern<<<unsigned(n_blocks), BS * NC, S::bytes(rows), s>>>(b);
+    launch_pdl(kern, unsigned(n_blocks), BS * NC, S::bytes(rows), s, b);
   }
 
   // trace + apply with the cross-block neighbour data prefetched (scalar problems)
