@@ -26,7 +26,7 @@
 // The geometry is stored by blocks of cells and copied with the rows, so that
 // nothing is waited for after the one staging (loading it face by face instead:
 // P2 FP64, three components 117 us, neighbours from global memory too 115 us,
-// staged 86 us).  The faces come first, then the cell term, which keeps the live
+// staged 80 us).  The faces come first, then the cell term, which keeps the live
 // values to about 50.  What is left for P2 FP64, three components: shared-memory
 // wavefronts 64 %, issue slots 46 %, FP64 pipe 40 % busy; in FP32 the issue slots
 // (72 %).  Persistent CTAs that copy the next block during the arithmetic were not
@@ -139,7 +139,7 @@ struct FusedShape {
   static constexpr int NG = 22 + (MASS ? 1 : 0);
   static constexpr int GEO = NG * BS * int(sizeof(T)) + 4 * BS * 2;  // bytes, a multiple of 16
   static_assert(GEO % 16 == 0, "blocks of whole 16-byte units");
-  static __host__ __device__ size_t bytes(int rows) { return GEO + size_t(rows) * US * sizeof(T); }
+  static __host__ __device__ size_t bytes(int rows) { return GEO + size_t(rows) * US * sizeof(T) + size_t(rows - BS) * 4; }
 };
 template <typename T>
 struct alignas(2 * sizeof(T)) Vec2 {
@@ -208,8 +208,36 @@ __host__ __device__ constexpr int dg_fused_min_ctas() {
   return sizeof(T) == 8 ? (P == 1 ? (NC == 1 ? 8 : 5) : (NC == 1 ? 4 : 3)) : (P == 1 ? (NC == 1 ? 12 : 6) : (NC == 1 ? 8 : 5));
 }
 
+// Rows of the outer neighbours of a block (at most 4 per cell): every index is
+// requested at once, ahead of the copies that need none of them, and goes
+// through shared memory to the threads that copy the rows.  Against a load per
+// copied value ahead of its copy (B200, 45 x 38 x 31 hexes): P2 FP64, three
+// components 85.5 -> 79.5 us, P1 37.9 -> 32.6, scalar P2 27.8 -> 25.5, scalar P2 FP32
+// 17.0 -> 16.2.  Padding the lists to one length, which saves the wait for their
+// beginnings, gave another 1 %: not kept.
+template <int BS, int THREADS>
+struct OuterRows {
+  static constexpr int N = (4 * BS + THREADS - 1) / THREADS;
+  int32_t v[N];
+  __device__ __forceinline__ void load(const int32_t* ext, int ne) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int r = int(threadIdx.x) + i * THREADS;
+      v[i] = r < ne ? __ldg(ext + r) : 0;
+    }
+  }
+  __device__ __forceinline__ void publish(int32_t* s, int ne) const {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int r = int(threadIdx.x) + i * THREADS;
+      if (r < ne) s[r] = v[i];
+    }
+    __syncthreads();
+  }
+};
+
 template <int P, int NC, bool MASS, int BS, typename T, int MINB>
-__global__ void __launch_bounds__(BS* NC, MINB) dg_fused_kernel(const __grid_constant__ DGBatch<T> batch) {
+__global__ void __launch_bounds__(BS* NC, MINB) dg_fused_kernel(const __grid_constant__ DGBatch<T> batch, int rows) {
   using O = gen::Ops<P>;
   using S = FusedShape<P, NC, MASS, BS, T>;
   constexpr int K = O::K, KQ = O::KQ, THREADS = BS * NC;
@@ -225,6 +253,9 @@ __global__ void __launch_bounds__(BS* NC, MINB) dg_fused_kernel(const __grid_con
   const int t = threadIdx.x, cell = t % BS, comp = t / BS;
   // ---- geometry and rows into shared memory
   const int32_t e0 = __ldg(pr.ext_begin + lb), ne = __ldg(pr.ext_begin + lb + 1) - e0;
+  int32_t* sx = reinterpret_cast<int32_t*>(su + rows * S::US);  // [rows - BS] outer neighbours
+  OuterRows<BS, THREADS> outer;
+  outer.load(pr.ext + e0, ne);
   {
     const unsigned char* g = pr.fgeo + lb * S::GEO;
     for (int e = t; e < S::GEO / 16; e += THREADS) cp_async_bytes<16>(smem_raw + 16 * e, g + 16 * e);
@@ -234,17 +265,19 @@ __global__ void __launch_bounds__(BS* NC, MINB) dg_fused_kernel(const __grid_con
     const T* own = pr.src + c0 * S::U;
     for (int e = t; e < nloc * S::CH; e += THREADS)
       cp_async_bytes<S::CB>(su + (e / S::CH) * S::US + 2 * (e % S::CH), own + 2 * e);
+    outer.publish(sx, ne);
 #pragma unroll 4
     for (int e = t; e < ne * S::CH; e += THREADS) {
       const int r = e / S::CH, v = e % S::CH;
-      cp_async_bytes<S::CB>(su + (BS + r) * S::US + 2 * v, pr.src + int64_t(__ldg(pr.ext + e0 + r)) * S::U + 2 * v);
+      cp_async_bytes<S::CB>(su + (BS + r) * S::US + 2 * v, pr.src + int64_t(sx[r]) * S::U + 2 * v);
     }
   } else {
     for (int e = t; e < nloc * S::U; e += THREADS)
       cp_async_bytes<sizeof(T)>(su + (e / S::U) * S::US + e % S::U, pr.src + c0 * S::U + e);
+    outer.publish(sx, ne);
     for (int e = t; e < ne * S::U; e += THREADS) {
       const int r = e / S::U, v = e % S::U;
-      cp_async_bytes<sizeof(T)>(su + (BS + r) * S::US + v, pr.src + int64_t(__ldg(pr.ext + e0 + r)) * S::U + v);
+      cp_async_bytes<sizeof(T)>(su + (BS + r) * S::US + v, pr.src + int64_t(sx[r]) * S::U + v);
     }
   }
   cp_async_commit();

@@ -369,7 +369,7 @@ class DGOperator final : public Operator {
     auto kern = dg_fused_kernel<P, NC, MASS, BS, T, dg_fused_min_ctas<P, NC, T>()>;
     // at most BS cells with four outer neighbours each
     opt_in_smem(kern, S::bytes(5 * BS), conf);
-    launch_pdl(kern, unsigned(n_blocks), BS * NC, S::bytes(rows), s, b);
+    launch_pdl(kern, unsigned(n_blocks), BS * NC, S::bytes(rows), s, b, rows);
   }
 
   // trace + apply with the cross-block neighbour data prefetched (scalar problems)
