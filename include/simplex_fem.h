@@ -80,8 +80,8 @@ typedef struct fem_op_params {
   double mass_coefficient; /* FEM_HELMHOLTZ: factor of the mass term (reference: 1e5) */
   int32_t n_components;    /* FEM_HELMHOLTZ: number of fields (reference: 3); others: 1 */
   int32_t penalty;         /* FEM_DG: enum fem_penalty */
-  int32_t kernel_variant;  /* 0: tuned default; DG/Helmholtz: 1 thread per cell x128 cells per
-                              CTA (P1, P2: single pass, thread per cell and component), 2 thread per cell x64, 3 warp roles x32, 4 thread per cell
+  int32_t kernel_variant;  /* 0: tuned default; DG/Helmholtz: 1 one launch, thread per cell and
+                              component (vmult_phase: thread per cell x128), 2 thread per cell x64, 3 warp roles x32, 4 thread per cell
                               x64 with results in registers (scalar) and 8 CTAs per SM, 5 thread
                               per cell x64 with 5 CTAs per SM; CG: 1 thread per
                               cell, 2 thread per Kuhn hex (6 tets, one atomic per distinct

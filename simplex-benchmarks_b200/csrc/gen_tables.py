@@ -632,6 +632,30 @@ def write_kernels(data, path):
         body = []
         emit_program(body, prog, 3 * KQ, lambda r: f"y({r})", lambda c: f"h[{c}]", True)
         fn("y(i) += (sum_a D_a^T h_a)_i", f"gradTInto_P{p}(const T (&h)[{3*KQ}], F&& y)", body)
+        # seen from a face: nodes by layers from the face (layer l: l nodes' worth of
+        # the opposite vertex), each layer in canonical face order, vertices (v0, v1,
+        # v2, opposite); the same formulas then hold for all four faces
+        lat_side = sorted(lat, key=lambda a: (a[3], -a[0], -a[1]))
+        d["SIDE"] = []
+        for f in range(4):
+            v = [x for x in range(4) if x != f] + [f]
+            rows = []
+            for a in lat_side:
+                b = [0, 0, 0, 0]
+                for k in range(4):
+                    b[v[k]] = a[k]
+                rows.append(lat.index(tuple(b)))
+            assert rows[:NF] == d["FN"][f]
+            d["SIDE"].append(rows)
+        # derivatives along v_w - opposite vertex at the P_{p-1} face nodes (face 3)
+        side = d["SIDE"][3]
+        along = []
+        for w in range(3):
+            for m in d["FNQ"][3]:
+                row = [(d["D"][w - 1][m][i] if w else Fr(0)) - d["D"][2][m][i] for i in range(K)]
+                along.append([row[side[i]] for i in range(K)])
+        product_fn(f"g[w*{NFQ}+m] = derivative along v_w - o at face node m, from a cell's values in side order",
+                   f"sideGrad_P{p}(const T* s, T* g)", along, lambda r: f"g[{r}]", lambda c: f"s[{c}]")
         # the same three row by row, for the CG kernels that run out of registers
         # before they run out of arithmetic (see cg_local_apply)
         body = []
@@ -760,6 +784,9 @@ def write_kernels(data, path):
         L.append(f"  static __host__ __device__ __forceinline__ constexpr int faceq_pos(int f, int m) {{ return faceq_pos_P{p}(f, m); }}")
         cases = " ".join(f"case {f*NF+i}: return {d['FN'][f][i]};" for f in range(4) for i in range(NF))
         L.append(f"  static __host__ __device__ __forceinline__ constexpr int fn(int f, int i) {{ switch (f * {NF} + i) {{ {cases} }} return 0; }}")
+        L.append(f"  template <class T> static __device__ __forceinline__ void sideGrad(const T* s, T* g) {{ sideGrad_P{p}(s, g); }}")
+        cases = " ".join(f"case {f*K+i}: return {d['SIDE'][f][i]};" for f in range(4) for i in range(K))
+        L.append(f"  static __host__ __device__ __forceinline__ constexpr int side(int f, int i) {{ switch (f * {K} + i) {{ {cases} }} return 0; }}")
         # Kuhn hex: lattice offset (x, y, z in 0..p) of node i of tet q.  Tet q walks
         # the hex edges in axis order KUHN[q], which is also the order of its
         # (ascending) vertices.

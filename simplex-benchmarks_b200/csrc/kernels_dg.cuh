@@ -60,11 +60,14 @@ struct DGProblem {
   const T* geo;       // [n_geo][n_cells]
   const int32_t* nb;  // [4][n_cells]
   const int8_t* nbf;  // [4][n_cells]
-  // single-pass form (kernels_dg_fused.cuh), P1 and P2 only
-  const unsigned char* fgeo;  // geometry by blocks of cells (FusedShape)
+  // single-launch forms (kernels_dg_fused.cuh, kernels_dg_fused3.cuh)
+  const unsigned char* fgeo;  // geometry by blocks of cells
   const int32_t* ext_begin;   // [blocks + 1] outer neighbours of every block
   const int32_t* ext;
   int32_t n_ext;              // most of a block (host)
+  const int32_t* face_begin;  // P3: [blocks + 1] outer faces of every block
+  const void* outer;          // P3: OuterFace<T>
+  int32_t n_outer;            // most of a block (host)
   const T* src;       // [n_cells][NC][K]
   T* dst;
   T* Q;               // [n_cells][4][NC][NFQ], or block-major (see dg_trace_blk_kernel)

@@ -11,6 +11,7 @@
 #include "kernels_dg2.cuh"
 #include "kernels_dg3.cuh"
 #include "kernels_dg_fused.cuh"
+#include "kernels_dg_fused3.cuh"
 #include "op_shapes.hpp"
 #include "operator.hpp"
 #include "operator_parts.hpp"
@@ -26,10 +27,13 @@ class DGOperator final : public Operator {
   DevBuf<T> d_geo;      // [6 + 4 + (mass?1:0)][n_cells]
   DevBuf<int32_t> d_nb; // [4][n_cells]
   DevBuf<int8_t> d_nbf; // [4][n_cells]
-  // P1 and P2, single-pass form (kernels_dg_fused.cuh)
+  // single-launch forms (kernels_dg_fused.cuh, kernels_dg_fused3.cuh)
   DevBuf<unsigned char> d_fgeo;  // geometry by blocks of cells
   DevBuf<int32_t> d_ext_begin, d_ext;  // outer neighbours of every block
   int n_ext = 0;            // most of a block
+  DevBuf<int32_t> d_face_begin;          // P3: outer faces of every block
+  DevBuf<OuterFace<T>> d_outer;
+  int n_outer = 0;
   DevBuf<T> d_Q;        // published face normal derivatives: [n_cells][4][NC][NFQ], or block-major
                         // (scalar problems, 1-thread-per-cell forms), for whole 128-cell blocks
   DevBuf<int> d_status; // timeouts of the bounded waits in the bulk-copy trace pass
@@ -108,26 +112,36 @@ class DGOperator final : public Operator {
       }
     d_nb.upload(nb);
     d_nbf.upload(nbf);
-    if (p <= 2) build_fused(mesh, geo);
+    build_fused(mesh, geo);
     d_Q.alloc(size_t((n_cells + kQB - 1) / kQB * kQB) * 4 * cfg.n_components * nfq_of(p));
     d_status.alloc(1);
     SFEM_CUDA(cudaMemset(d_status.p, 0, sizeof(int)));
   }
 
-  static int fused_block(int nc) { return nc == 1 ? dg_fused_cells<1>() : dg_fused_cells<3>(); }
+  // cells of a block of the single-launch form
+  int fused_block() const {
+    if (cfg.degree == 3) return cfg.n_components == 1 ? dg_fused3_cells<1>() : dg_fused3_cells<3>();
+    return cfg.n_components == 1 ? dg_fused_cells<1>() : dg_fused_cells<3>();
+  }
 
+  // Geometry, outer neighbours and (P3) outer faces by blocks of cells: FusedShape
+  // (P1, P2) and Fused3Shape (P3)
   void build_fused(const Mesh& mesh, const std::vector<T>& geo) {
-    const int64_t BS = fused_block(cfg.n_components), nblk = (n_cells + BS - 1) / BS;
-    const int NG = has_mass ? 23 : 22;  // FusedShape
-    const size_t block_bytes = size_t(NG) * BS * sizeof(T) + 4 * BS * sizeof(uint16_t);
+    const int64_t BS = fused_block(), nblk = (n_cells + BS - 1) / BS;
+    const bool p3 = cfg.degree == 3;
+    const int NG = (p3 ? 10 : 22) + (has_mass ? 1 : 0);
+    const size_t block_bytes = size_t(NG) * BS * sizeof(T) + 4 * BS * (p3 ? sizeof(uint32_t) : sizeof(uint16_t));
     std::vector<unsigned char> fg(block_bytes * nblk, 0);
     std::vector<std::vector<int32_t>> outer(nblk);
+    std::vector<std::vector<OuterFace<T>>> faces(p3 ? nblk : 0);
 #pragma omp parallel for schedule(static)
     for (int64_t b = 0; b < nblk; ++b) {
       const int64_t c0 = b * BS, c1 = std::min(n_cells, c0 + BS);
       T* g = reinterpret_cast<T*>(fg.data() + b * block_bytes);
-      uint16_t* code = reinterpret_cast<uint16_t*>(g + NG * BS);
-      std::fill(code, code + 4 * BS, kBoundary);
+      uint16_t* code = reinterpret_cast<uint16_t*>(g + NG * BS);    // P1, P2
+      uint32_t* code3 = reinterpret_cast<uint32_t*>(g + NG * BS);   // P3
+      if (p3) std::fill(code3, code3 + 4 * BS, kBoundary3);
+      else std::fill(code, code + 4 * BS, kBoundary);
       std::vector<int32_t>& ex = outer[b];
       for (int64_t cc = c0; cc < c1; ++cc)
         for (int f = 0; f < 4; ++f) {
@@ -138,39 +152,64 @@ class DGOperator final : public Operator {
       ex.erase(std::unique(ex.begin(), ex.end()), ex.end());
       for (int64_t cc = c0; cc < c1; ++cc) {
         for (int k = 0; k < 10; ++k) g[k * BS + cc - c0] = geo[size_t(k) * n_cells + cc];
-        if (has_mass) g[22 * BS + cc - c0] = geo[size_t(10) * n_cells + cc];
+        if (has_mass) g[(NG - 1) * BS + cc - c0] = geo[size_t(10) * n_cells + cc];
         for (int f = 0; f < 4; ++f) {
-          // J^-1 (2|F| n) of the neighbour on its side of the face, as the barycentric
-          // weights of the three face vertices (own values on the boundary, unread)
           const int32_t nbc = mesh.nb[4 * cc + f];
-          const int64_t o = nbc >= 0 ? nbc : cc;
-          const int of = nbc >= 0 ? mesh.nbf[4 * cc + f] : f;
-          double G[6], w[4] = {0, 0, 0, 0};
-          metric(cell_geometry(mesh, o), G);
-          const double M[3][3] = {{G[0], G[3], G[4]}, {G[3], G[1], G[5]}, {G[4], G[5], G[2]}};
-          for (int a = 0; a < 3; ++a) {
-            w[a + 1] = of == 0 ? M[a][0] + M[a][1] + M[a][2] : -M[a][of - 1];
-            w[0] -= w[a + 1];
-          }
-          for (int v = 0, k = 0; v < 4; ++v)
-            if (v != of) g[(10 + 3 * f + k++) * BS + cc - c0] = T(w[v]);
           if (nbc < 0) continue;
-          const int64_t row = nbc >= c0 && nbc < c1
-                                  ? nbc - c0
-                                  : BS + (std::lower_bound(ex.begin(), ex.end(), nbc) - ex.begin());
-          code[f * BS + cc - c0] = uint16_t(row << 2 | of);
+          const int of = mesh.nbf[4 * cc + f];
+          const bool in = nbc >= c0 && nbc < c1;
+          const int64_t row = in ? nbc - c0 : BS + (std::lower_bound(ex.begin(), ex.end(), nbc) - ex.begin());
+          // J^-1 (2|F| n) of the neighbour on its side of the face, as the barycentric
+          // weights of its three face vertices
+          T w[3];
+          if (!p3 || !in) {
+            double G[6], c[4] = {0, 0, 0, 0};
+            metric(cell_geometry(mesh, nbc), G);
+            const double M[3][3] = {{G[0], G[3], G[4]}, {G[3], G[1], G[5]}, {G[4], G[5], G[2]}};
+            for (int a = 0; a < 3; ++a) {
+              c[a + 1] = of == 0 ? M[a][0] + M[a][1] + M[a][2] : -M[a][of - 1];
+              c[0] -= c[a + 1];
+            }
+            for (int v = 0, k = 0; v < 4; ++v)
+              if (v != of) w[k++] = T(c[v]);
+          }
+          if (p3) {
+            uint32_t slot = 0;
+            if (!in) {
+              slot = uint32_t(faces[b].size());
+              OuterFace<T> o;
+              o.pad = T(0);
+              for (int k = 0; k < 3; ++k) o.w[k] = w[k];
+              o.code = uint32_t(row) | uint32_t(of) << 14;
+              faces[b].push_back(o);
+            }
+            code3[f * BS + cc - c0] = uint32_t(row) | uint32_t(of) << 14 | slot << 16;
+          } else {
+            for (int k = 0; k < 3; ++k) g[(10 + 3 * f + k) * BS + cc - c0] = w[k];
+            code[f * BS + cc - c0] = uint16_t(row << 2 | of);
+          }
         }
       }
     }
-    std::vector<int32_t> begin(nblk + 1, 0), ext;
+    std::vector<int32_t> begin(nblk + 1, 0), ext, fbegin(nblk + 1, 0);
+    std::vector<OuterFace<T>> all;
     for (int64_t b = 0; b < nblk; ++b) {
       n_ext = std::max(n_ext, int(outer[b].size()));
       ext.insert(ext.end(), outer[b].begin(), outer[b].end());
       begin[b + 1] = int32_t(ext.size());
+      if (p3) {
+        n_outer = std::max(n_outer, int(faces[b].size()));
+        all.insert(all.end(), faces[b].begin(), faces[b].end());
+        fbegin[b + 1] = int32_t(all.size());
+      }
     }
     d_ext_begin.upload(begin);
     d_fgeo.upload(fg);
     d_ext.upload(ext);
+    if (p3) {
+      d_face_begin.upload(fbegin);
+      d_outer.upload(all);
+    }
   }
 
   int status(bool clear) override {
@@ -189,6 +228,9 @@ class DGOperator final : public Operator {
     pr.ext_begin = d_ext_begin.p;
     pr.ext = d_ext.p;
     pr.n_ext = n_ext;
+    pr.face_begin = d_face_begin.p;
+    pr.outer = d_outer.p;
+    pr.n_outer = n_outer;
     pr.src = static_cast<const T*>(src);
     pr.dst = static_cast<T*>(dst);
     pr.Q = d_Q.p;
@@ -240,7 +282,7 @@ class DGOperator final : public Operator {
     const int nc = cfg.n_components;
     SFEM_REQUIRE(nc == 1 || nc == 3, FEM_ERR_ARG, "DG: n_components must be 1 or 3");
     SFEM_REQUIRE(n >= 1 && n <= kMaxBatch, FEM_ERR_ARG, "DG: 1..40 problems per launch");
-    const int variant = cfg.kernel_variant > 0 ? cfg.kernel_variant : default_variant(cfg.degree, nc);
+    const int variant = cfg.kernel_variant > 0 ? cfg.kernel_variant : default_variant(cfg.degree, nc, what);
 #define SFEM_DG_CASE(P, NC, MASS)                                                       \
   if (cfg.degree == P && nc == NC && mass == MASS) {                                    \
     run<P, NC, MASS>(probs, n, s, what, variant, status);                               \
@@ -254,16 +296,12 @@ class DGOperator final : public Operator {
     throw Error(FEM_ERR_ARG, "DG: unsupported degree/components combination");
   }
 
-  // kernel forms: 1 thread per cell, 128 cells per CTA (P1 and P2: one pass with a
-  // thread per cell and component); 2 thread per cell, 64
-  // cells per CTA; 3 warp roles, 32 cells per CTA
-  // (measured on B200: scalar P3 runs best register-capped at 64 cells per CTA,
-  // the 3-component forms at 128 cells per CTA)
-  // measured on B200 (DG P3 32^3, medians of 25 L2-flushed vmults): FP64
-  // 82.9 us with 128 cells per CTA against 85.0 us with 64; FP32 44.1 us with
-  // the results in registers and 8 CTAs per SM against 52.2 us; 128 cells per
-  // CTA otherwise
-  static int default_variant(int p, int nc) { return (nc == 1 && p == 3 && sizeof(T) == 4) ? 4 : 1; }
+  // kernel forms: 1 one launch with a thread per cell and component, its single
+  // phases with 128 cells per CTA; 2 thread per cell, 64 cells per CTA; 3 warp
+  // roles, 32 cells per CTA.  Single phases (vmult_phase) of scalar FP32 P3 run
+  // best with the results in registers and 8 CTAs per SM (B200, 32^3: 38 us for
+  // both against 44).
+  static int default_variant(int p, int nc, int what) { return (nc == 1 && p == 3 && sizeof(T) == 4 && what != 0) ? 4 : 1; }
 
   static DGBatch<T> make_batch(const DGProblem<T>* probs, int n, int bs, int64_t& n_blocks) {
     DGBatch<T> b;
@@ -372,6 +410,39 @@ class DGOperator final : public Operator {
     launch_pdl(kern, unsigned(n_blocks), BS * NC, S::bytes(rows), s, b, rows);
   }
 
+  // P3 in one launch pays except for scalar FP64 with most neighbours outside
+  // the block, where a CTA's shared memory holds five rows per cell and one CTA
+  // fits an SM (B200, DG P3, 24^3 hexes, us per vmult, one launch / two): cells by
+  // x-rows (1.3 outer faces per cell) FP64 22.4 / 29.5, FP32 14.4 / 18.3; cells in
+  // random order (4) FP64 45.4 / 38.4, FP32 26.6 / 44.7; 3 components FP64 168 /
+  // 186, FP32 65 / 117.  The FP64 lines through both points meet near 2.7.
+  template <int NC>
+  static bool fused3_pays(const DGProblem<T>* probs, int n) {
+    if (NC > 1 || sizeof(T) == 4) return true;
+    for (int i = 0; i < n; ++i)
+      if (probs[i].n_outer > 5 * dg_fused3_cells<NC>() / 2) return false;
+    return true;
+  }
+
+  // P3 in one launch (kernels_dg_fused3.cuh)
+  template <int NC, bool MASS>
+  static void run_fused3(const DGProblem<T>* probs, int n, cudaStream_t s) {
+    constexpr int BS = dg_fused3_cells<NC>();
+    using S = Fused3Shape<NC, MASS, BS, T>;
+    int64_t n_blocks = 0;
+    const DGBatch<T> b = make_batch(probs, n, BS, n_blocks);
+    int ne = 0, nf = 0;
+    for (int i = 0; i < n; ++i) {
+      ne = std::max(ne, probs[i].n_ext);
+      nf = std::max(nf, probs[i].n_outer);
+    }
+    static std::atomic<uint64_t> conf{0};
+    auto kern = dg_fused3_kernel<NC, MASS, BS, T, dg_fused3_min_ctas<NC, T>()>;
+    // at most BS cells with four outer neighbours each
+    opt_in_smem(kern, S::bytes(4 * BS, 4 * BS), conf);
+    launch_pdl(kern, unsigned(n_blocks), BS * NC, S::bytes(ne, nf), s, b, ne, nf);
+  }
+
   // trace + apply with the cross-block neighbour data prefetched (scalar problems)
   template <int P, int BS, int XCAP>
   static void run_xp(const DGProblem<T>* probs, int n, cudaStream_t s, int what) {
@@ -431,6 +502,8 @@ class DGOperator final : public Operator {
       // P1 and P2: one pass (B200, 45 x 38 x 31 hexes: see kernels_dg_fused.cuh); the
       // two passes below are what vmult_phase runs
       if constexpr (P <= 2) run_fused<P, NC, MASS>(probs, n, s);
+    } else if (variant == 1 && what == 0 && fused3_pays<NC>(probs, n)) {
+      if constexpr (P == 3) run_fused3<NC, MASS>(probs, n, s);
     } else if (variant == 1) {
       // scalar problems: the apply pass loads its geometry and src rows while
       // the trace pass finishes (B200, DG P3 FP64 32^3: 68.5 -> 64.5 us per vmult)
