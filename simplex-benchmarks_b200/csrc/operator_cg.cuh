@@ -13,6 +13,7 @@
 #include "op_shapes.hpp"
 #include "operator.hpp"
 #include "operator_cg_block.hpp"
+#include "operator_cg_patch.hpp"
 #include "operator_parts.hpp"
 
 namespace sfem {
@@ -94,6 +95,8 @@ class CGOperator final : public Operator {
 
   // 4 x 4 x 4-hex blocks of cg_block_kernel; empty on meshes that are no Kuhn boxes
   CGBlocks<T, 1> blocks;
+  // patches of cells of cg_patch_kernel, where a thread per cell is the default
+  CGPatches<T, 1> patches;
 
   // cube-block tables of cg_cube_kernel (blocks of 64 hexes = 384 tets)
   DevBuf<int16_t> d_tmapv, d_cslot8[3];
@@ -516,6 +519,7 @@ class CGOperator final : public Operator {
     build_hex_tables(mesh, dofs, geo);
     build_cube_tables(dofs);
     blocks.build(mesh, cfg.degree, dofs.cell_dofs, dofs.constrained, geo);
+    if (default_variant() == 1) patches.build(cfg.degree, K, n_cells, dofs.cell_dofs, dofs.constrained);
     if (cfg.weak_bc) build_weak_boundary(mesh);
     d_status.alloc(1);
     SFEM_CUDA(cudaMemset(d_status.p, 0, sizeof(int)));
@@ -648,7 +652,8 @@ class CGOperator final : public Operator {
   // Variant 0: forms 3 (blocks or cubes) and 1 (thread per cell), the latter on
   // meshes with fewer blocks than SMs, where most SMs would idle (P2 FP64 16^3 5.0
   // against 7.8 us, 24^3 equal, 32^3 13.9 against 8.9 us), and for P3 FP64 without
-  // whole cubes (37 x 41 x 35 hexes: 41.5 us, per hex 49.5 us).
+  // whole cubes (37 x 41 x 35 hexes: 41.5 us, per hex 49.5 us).  Where 1 is the
+  // default and the mesh has enough patches (CGPatches), 1 runs cg_patch_kernel.
   int default_variant() const {
     const bool cubes = cube_NB && n_blocks >= 2 * 148;
     if (cfg.degree <= 2) return blocks.n_blocks >= 148 ? 3 : 1;
@@ -708,6 +713,10 @@ class CGOperator final : public Operator {
       SFEM_CUDA(cudaGetLastError());
       return;
     }
+    if (v == 1 && patches.n_patches) {
+      patches.launch(cfg.degree, d_geo.p, x, d, d_constrained.n, d_constrained.p, s);
+      return;
+    }
     const int64_t n = std::max<int64_t>(n_cells, int64_t(d_constrained.n));
     const unsigned grid = blocks_for(n, 128);
     switch (cfg.degree) {
@@ -764,7 +773,7 @@ class CGOperator final : public Operator {
 // (index 3 g + comp), as the reference's components-batched CG operator
 // (CG/components_batched/application.cc:778-1611, FESystem of dim
 // FE_SimplexP).  Homogeneous Dirichlet on every component of the boundary
-// nodes.  Thread per cell, or cg_block_kernel on Kuhn boxes.
+// nodes.  cg_block_kernel on Kuhn boxes, else cg_patch_kernel or a thread per cell.
 template <typename T>
 class CGVectorOperator final : public Operator {
  public:
@@ -775,6 +784,7 @@ class CGVectorOperator final : public Operator {
   int64_t n_nodes = 0;
   std::vector<int32_t> node_dofs;  // [n_cells][K]
   CGBlocks<T, NC> blocks;          // 4 x 4 x 4-hex blocks (Kuhn boxes)
+  CGPatches<T, NC> patches;        // patches of cells elsewhere
 
   CGVectorOperator(const Mesh& mesh, const OpConfig& c) {
     cfg = c;
@@ -816,7 +826,12 @@ class CGVectorOperator final : public Operator {
     d_geo.upload(geo);
     d_constrained.upload(cl);
     blocks.build(mesh, cfg.degree, dofs.cell_dofs, dofs.constrained, geo);
+    // P3 FP64 keeps the thread per cell: 44 x 40 x 36 hexes 130 us, by patches 137 to 160
+    if (!block_form() && (cfg.degree <= 2 || sizeof(T) == 4))
+      patches.build(cfg.degree, K, n_cells, dofs.cell_dofs, dofs.constrained);
   }
+  // P3 FP64: the block form is slower than a thread per cell (48^3 392 against 226 us)
+  bool block_form() const { return blocks.n_blocks >= 148 && (cfg.degree <= 2 || sizeof(T) == 4); }
 
   void vmult(void* dst, const void* src, cudaStream_t s) override {
     vmult_phase(dst, src, 1, s);
@@ -830,9 +845,12 @@ class CGVectorOperator final : public Operator {
       SFEM_CUDA(cudaMemsetAsync(d, 0, sizeof(T) * m, s));
       return;
     }
-    // P3 FP64: the block form is slower than a thread per cell (48^3 392 against 226 us)
-    if (cfg.kernel_variant == 0 && blocks.n_blocks >= 148 && (cfg.degree <= 2 || sizeof(T) == 4)) {
+    if (cfg.kernel_variant == 0 && block_form()) {
       blocks.launch(cfg.degree, x, d, d_constrained.n, d_constrained.p, s);
+      return;
+    }
+    if (patches.n_patches) {
+      patches.launch(cfg.degree, d_geo.p, x, d, d_constrained.n, d_constrained.p, s);
       return;
     }
     const unsigned grid = blocks_for(std::max<int64_t>(n_cells, int64_t(d_constrained.n)), 128);
