@@ -196,14 +196,18 @@ def check(status):
         raise FemError(status, lib().fem_last_error_string().decode())
 
 
+# Handles go to C as plain integers, which ctypes converts faster than c_void_p
+# objects, and the current stream comes without a Stream object around it: a small
+# product's call is host work (P2 16^3, B200: 10.2 -> 6.4 us).
 def _stream_ptr(stream=None):
+    if stream is not None:
+        return stream.cuda_stream
     import torch
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return C.c_void_p(s.cuda_stream)
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _ptr(t):
-    return C.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 class Mesh:
