@@ -972,7 +972,11 @@ class MultigridImpl final : public Multigrid {
     const double theta = 0.5 * (L.lmax + L.lmin), delta = 0.5 * (L.lmax - L.lmin);
     double rho = delta / theta;
     if (zero_init) {
-      launch_pdl(cheb_first_zero<T>, g, 256, 0, s, m, T(1.0 / theta), L.inv_diag.p, b, L.d.p, x);
+      if (in_packs(m, b, x))
+        launch_pdl(cheb_first_zero<T, kPack>, grid_for(m / kPack), 256, 0, s, m, T(1.0 / theta), L.inv_diag.p, b,
+                   L.d.p, x);
+      else
+        launch_pdl(cheb_first_zero<T, 1>, g, 256, 0, s, m, T(1.0 / theta), L.inv_diag.p, b, L.d.p, x);
     } else {
       product(L, x, s);
       cheb<true>(L, T(0), T(1.0 / theta), b, x, s);
@@ -993,13 +997,18 @@ class MultigridImpl final : public Multigrid {
     if (L.clear_t) L.op->vmult_zeroed(L.t.p, x, s);
     else L.op->vmult(L.t.p, x, s);
   }
+  // values moved at once (b and x can be a caller's; the level's own vectors are aligned)
+  static constexpr int kPack = 16 / sizeof(T);
   template <bool FIRST>
   void cheb(Level& L, T f1, T f2, const T* b, T* x, cudaStream_t s) {
     const int64_t m = L.op->m;
     if (L.clear_t)
-      launch_pdl(cheb_step<T, FIRST, true>, grid_for(m), 256, 0, s, m, f1, f2, L.inv_diag.p, b, L.t.p, L.d.p, x, 0);
+      launch_pdl(cheb_step<T, FIRST, true, 1>, grid_for(m), 256, 0, s, m, f1, f2, L.inv_diag.p, b, L.t.p, L.d.p, x, 0);
+    else if (in_packs(m, b, x))
+      launch_pdl(cheb_step<T, FIRST, false, kPack>, grid_for(m / kPack), 256, 0, s, m, f1, f2, L.inv_diag.p, b,
+                 L.t.p, L.d.p, x, 0);
     else
-      launch_pdl(cheb_step<T, FIRST, false>, grid_for(m), 256, 0, s, m, f1, f2, L.inv_diag.p, b, L.t.p, L.d.p, x, 0);
+      launch_pdl(cheb_step<T, FIRST, false, 1>, grid_for(m), 256, 0, s, m, f1, f2, L.inv_diag.p, b, L.t.p, L.d.p, x, 0);
   }
   // r = b - t, and z = 0 (z may be null)
   void residual(Level& L, const T* b, T* r, T* z, int64_t nz, cudaStream_t s) {
