@@ -446,7 +446,8 @@ int fem_batch_set_kernel_variant(fem_batch* batch, int32_t variant);
  * (median of `reps` launches after 2 warm-ups, on zero input), keeps the
  * fastest and returns it in *variant.  us[8] receives the median time per
  * variant 1..8 (0 = not a candidate; CG's approximate TF32 variant 4 is
- * never a candidate, and CG's cube variant 3 is timed as 5, 6 and 7).  With use_cache != 0 a choice recorded for
+ * never a candidate; CG's variant 3 is timed where it is the block form and
+ * the default, its cube schedules as 5, 6 and 7).  With use_cache != 0 a choice recorded for
  * the same (kind, degree, precision, components, log2 cells, GPU name) is
  * applied without timing (*cached = 1).  fem_autotune_cache sets a file that
  * keeps the choices across processes (JSON lines; NULL = memory only).

@@ -746,6 +746,7 @@ class CGOperator final : public Operator {
   }
 
   const int32_t* device_dof_table() const override { return d_dofs.p; }
+  bool block_default() const override { return blocks.n_blocks && use_blocks() && default_variant() == 3; }
   const BlockView* block_view() const override { return blocks.view.n_blocks ? &blocks.view : nullptr; }
 
   void element_matrices(void* out, cudaStream_t s) override {
@@ -832,6 +833,7 @@ class CGVectorOperator final : public Operator {
   }
   // P3 FP64: the block form is slower than a thread per cell (48^3 392 against 226 us)
   bool block_form() const { return blocks.n_blocks >= 148 && (cfg.degree <= 2 || sizeof(T) == 4); }
+  bool block_default() const override { return block_form(); }
 
   void vmult(void* dst, const void* src, cudaStream_t s) override {
     vmult_phase(dst, src, 1, s);
@@ -845,7 +847,7 @@ class CGVectorOperator final : public Operator {
       SFEM_CUDA(cudaMemsetAsync(d, 0, sizeof(T) * m, s));
       return;
     }
-    if (cfg.kernel_variant == 0 && block_form()) {
+    if ((cfg.kernel_variant == 0 || cfg.kernel_variant == 3) && block_form()) {
       blocks.launch(cfg.degree, x, d, d_constrained.n, d_constrained.p, s);
       return;
     }
