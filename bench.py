@@ -45,7 +45,7 @@ WORKLOAD = "DG SIPG Poisson vmult, P3 on 32^3 x 6 Kuhn tets (196,608 cells, 3,93
 # workload: dram__bytes_read.sum + dram__bytes_write.sum of an ncu capture
 # (profiles/dg_apply_kernel_p3_fp64_32cube.md)
 VMULT_KERNEL = "dg_fused3_kernel<1,false,128,double,2>"
-VMULT_TRAFFIC_BYTES = 66.25e6
+VMULT_TRAFFIC_BYTES = 66.25e6  # captured with blocks of 64 cells
 
 
 def parse():
