@@ -84,7 +84,8 @@ typedef struct fem_op_params {
                               component (vmult_phase: thread per cell x128), 2 thread per cell x64, 3 warp roles x32, 4 thread per cell
                               x64 with results in registers (scalar) and 8 CTAs per SM, 5 thread
                               per cell x64 with 5 CTAs per SM; CG: 1 thread per
-                              cell, 2 thread per Kuhn hex (6 tets, one atomic per distinct
+                              cell (by patches of consecutive cells on larger meshes where 1
+                              is the default), 2 thread per Kuhn hex (6 tets, one atomic per distinct
                               DoF), 3 CTA per 4x4x4 hexes (stores for interior DoFs: a thread
                               per hex, or per tet for P3 FP64 and small P3 FP32 meshes); each
                               falls back to the next simpler form where the mesh lacks the
