@@ -78,7 +78,7 @@ LearnedSmoother::LearnedSmoother(uint64_t seed) {
   m_.alloc(NP);
   v_.alloc(NP);
   g_.alloc(NP);
-  loss_.alloc(1);
+  sums_.alloc(NP + 1);
   wb_.alloc(NP);
   status_.alloc(1);
   SFEM_CUDA(cudaMemset(status_.p, 0, sizeof(int)));
@@ -181,25 +181,27 @@ void LearnedSmoother::launch_gradient(const float* X, const float* Y, int n, flo
                                    int(mlpg::Shape<2>::BYTES)));
   });
   SFEM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  SFEM_CUDA(cudaMemsetAsync(grad, 0, sizeof(float) * NP, s));
-  if (!accumulate_loss) SFEM_CUDA(cudaMemsetAsync(loss_.p, 0, sizeof(double), s));
+  // the sums, then the loss
+  SFEM_CUDA(cudaMemsetAsync(sums_.p, 0, sizeof(double) * (accumulate_loss ? NP : NP + 1), s));
   const GradPlan p = mlp_grad_plan(n, sms);
   const float inv = 1.0f / float(n);
   if (p.spt == 1)
-    mlp_grad_kernel<1><<<p.grid, mlpg::THREADS, mlpg::Shape<1>::BYTES, s>>>(n, X, Y, wb_.p, grad, loss_.p, inv);
+    mlp_grad_kernel<1><<<p.grid, mlpg::THREADS, mlpg::Shape<1>::BYTES, s>>>(n, X, Y, wb_.p, sums_.p, sums_.p + NP, inv);
   else
-    mlp_grad_kernel<2><<<p.grid, mlpg::THREADS, mlpg::Shape<2>::BYTES, s>>>(n, X, Y, wb_.p, grad, loss_.p, inv);
+    mlp_grad_kernel<2><<<p.grid, mlpg::THREADS, mlpg::Shape<2>::BYTES, s>>>(n, X, Y, wb_.p, sums_.p, sums_.p + NP, inv);
   SFEM_CUDA(cudaGetLastError());
+  launch_pdl(mlp_grad_round_kernel, (NP + 255) / 256, 256, 0, s, sums_.p, grad);
 }
 
 double LearnedSmoother::read_loss(cudaStream_t s) {
   double h = 0;
-  SFEM_CUDA(cudaMemcpyAsync(&h, loss_.p, sizeof(double), cudaMemcpyDeviceToHost, s));
+  SFEM_CUDA(cudaMemcpyAsync(&h, sums_.p + NP, sizeof(double), cudaMemcpyDeviceToHost, s));
   SFEM_CUDA(cudaStreamSynchronize(s));
   return h;
 }
 
 double LearnedSmoother::gradient(const float* X, const float* Y, int n, float* grad, cudaStream_t s) {
+  std::lock_guard<std::mutex> lock(sums_mutex_);  // until the loss is read: the sums are the handle's
   launch_gradient(X, Y, n, grad, false, s);
   return read_loss(s);
 }
@@ -226,6 +228,7 @@ TrainStats LearnedSmoother::train(const float* X, const float* Y, int n, int epo
                                   uint64_t seed) {
   using D = MLPDims;
   SFEM_REQUIRE(n > 0 && epochs > 0 && batch > 0, FEM_ERR_ARG, "mlp: bad training parameters");
+  std::lock_guard<std::mutex> lock(sums_mutex_);
   const auto t0 = std::chrono::steady_clock::now();
   TrainStats st;
   st.samples = n;

@@ -6,6 +6,7 @@
 #include <cstdint>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -72,11 +73,13 @@ class LearnedSmoother {
   };
   Bound& bind(const Operator& op);
   void round_weights(cudaStream_t s);
-  // gradient of the batch into grad and its loss (mean) into loss_, or added to it; no synchronisation
+  // gradient of the batch into grad and its loss (mean) into sums_[NP], or added to it; no
+  // synchronisation, the caller holds sums_mutex_ until read_loss
   void launch_gradient(const float* X, const float* Y, int n, float* grad, bool accumulate_loss, cudaStream_t s);
   double read_loss(cudaStream_t s);
   DevBuf<float> w_, m_, v_, g_;
-  DevBuf<double> loss_;
+  DevBuf<double> sums_;  // [NP] gradient sums, loss
+  std::mutex sums_mutex_;
   DevBuf<__nv_bfloat16> wb_;
   DevBuf<int> status_;
   bool tensor_cores_ = true;

@@ -9,21 +9,27 @@
 // neighbouring outputs of SPT samples (or a 4 x 4 block of a weight gradient)
 // and a warp's reads are broadcasts or contiguous rows without bank conflicts
 // (row strides of 68 and 36 words).  The weight gradients stay in registers
-// over all tiles of the CTA and leave once, as coalesced atomic additions (a
-// workspace of one row per CTA and a second reducing launch would be
-// reproducible bit for bit, but its allocation costs 3 ms on the first call).
+// over all tiles of the CTA and leave once, as coalesced atomic additions in FP64
+// that a second small launch rounds.  Added in FP32, one CTA's sums after another onto
+// the same total (128 CTAs for 2048 samples), the gradient's error against 64 bits is
+// 1.6e-7 at 2048 and 2.2e-7 at 8192 samples; so it is 3e-8 at both, for 1.3 us of a
+// call.  Eight or four CTAs of a cluster adding pairwise before an FP32 addition leave
+// 6e-8 and 8e-8, but 16 clusters of eight or more than 33 of four do not fit with one
+// CTA per SM (51 us a call).  A workspace of one row per CTA would be reproducible bit
+// for bit, but its allocation costs 3 ms on the first call.
 //
 // The kernel is bound by shared-memory reads (about 9 wavefronts for 16
 // multiply-adds of a warp) and by the latency of the eight products of a tile;
 // small batches are given one 16-sample tile per CTA to fill the SMs.  Measured
 // on B200, the whole call with its host read of the loss: 2048 samples (the
-// default batch) 44 us, 32,000 samples 109 us, against 13.3 and 13.8 ms for a
+// default batch) 42 us, 32,768 samples 103 us, against 13.1 and 13.7 ms for a
 // thread per sample with shared-memory atomics for every product.
 #pragma once
 #include <cuda_bf16.h>
 
 #include "mlp.cuh"
 #include "mlp_dims.hpp"
+#include "pdl.cuh"
 
 namespace sfem {
 namespace mlpg {
@@ -86,11 +92,11 @@ __device__ __forceinline__ void product(const float* M, const float* v, int col,
 
 }  // namespace mlpg
 
-// grad [NPARAM] and loss are zero on entry (loss: or a running sum)
+// sums [NPARAM] and loss are zero on entry (loss: or a running sum)
 template <int SPT>
 __global__ void __launch_bounds__(mlpg::THREADS, 2)
     mlp_grad_kernel(int n, const float* __restrict__ X, const float* __restrict__ Y,
-                    const __nv_bfloat16* __restrict__ wb, float* __restrict__ grad, double* __restrict__ loss,
+                    const __nv_bfloat16* __restrict__ wb, double* __restrict__ sums, double* __restrict__ loss,
                     float inv_batch) {
   using D = MLPDims;
   using namespace mlpg;
@@ -234,7 +240,18 @@ __global__ void __launch_bounds__(mlpg::THREADS, 2)
   for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
   if ((t & 31) == 0) atomicAdd(loss, double(lsum) * double(inv_batch));
   __syncthreads();
-  for (int i = t; i < D::NPARAM; i += THREADS) atomicAdd(grad + i, row[i]);
+  // every CTA begins elsewhere, so that they do not queue at the same addresses
+  constexpr int CH = (D::NPARAM + THREADS - 1) / THREADS;
+  for (int k = 0; k < CH; ++k) {
+    const int i = int((blockIdx.x + k) % CH) * THREADS + t;
+    if (i < D::NPARAM) atomicAdd(sums + i, double(row[i]));
+  }
+}
+
+__global__ void mlp_grad_round_kernel(const double* sums, float* grad) {
+  pdl_enter();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < MLPDims::NPARAM) grad[i] = float(sums[i]);
 }
 
 }  // namespace sfem
