@@ -107,7 +107,7 @@ void tune_set_cache_file(const std::string& path) {
 TuneResult autotune(Operator& op, int reps, bool use_cache) {
   TuneResult res;
   std::vector<int> cand = tune_candidates(op.cfg);
-  if (op.block_default() && std::find(cand.begin(), cand.end(), 3) == cand.end()) cand.push_back(3);
+  if (op.block_form() && std::find(cand.begin(), cand.end(), 3) == cand.end()) cand.push_back(3);
   res.us.assign(8, 0.0);
   const std::string key = tune_key(op.cfg, op.n_cells);
   if (use_cache) {

@@ -103,8 +103,9 @@ class Operator {
   virtual const int32_t* device_dof_table() const { return nullptr; }
   // CG on a Kuhn box: its blocks (nullptr: none)
   virtual const BlockView* block_view() const { return nullptr; }
-  // the block form (CG variant 3) is the default here: the autotuner times it too
-  virtual bool block_default() const { return false; }
+  // CG variant 3 is the block form here and has a block for every SM: the autotuner
+  // times it too
+  virtual bool block_form() const { return false; }
   // Device scratch one vmult needs (DG: the published face traces; CG: none).
   virtual size_t scratch_bytes() const { return 0; }
   // vmult with the scratch supplied by the caller instead of the operator's own.

@@ -640,24 +640,22 @@ class CGOperator final : public Operator {
     SFEM_CUDA(cudaGetLastError());
   }
 
-  // Block form (cg_block_kernel) or thread-per-tet cube kernel, where both apply.
-  // P1 and P2: always the block form.  P3 FP32: the block form once its blocks fill
-  // the SMs more than half (64 threads walk a whole block, 15 us: 32^3 15.8 against
-  // 17.4 us, but 24^3 15.6 against 10.4 us) or where there are no whole cubes.  P3
-  // FP64 (two resident CTAs of 64 threads): never (64^3 177 against 143 us).
+  // Variant 3: block form (cg_block_kernel) or thread-per-tet cube kernel, where both
+  // apply.  P1 and P2: always the block form.  P3 FP32: the block form where it pays or
+  // there are no whole cubes (a wave of blocks takes 15 us: 36^3 28.1, cubes 23.6 us).
   bool use_blocks() const {
-    if (cfg.degree <= 2) return true;
-    return sizeof(T) == 4 && (!cube_NB || blocks.n_blocks >= 400);
+    return blocks.n_blocks && (cfg.degree <= 2 || !cube_NB || blocks.pays(cfg.degree));
   }
-  // Variant 0: forms 3 (blocks or cubes) and 1 (thread per cell), the latter on
-  // meshes with fewer blocks than SMs, where most SMs would idle (P2 FP64 16^3 5.0
-  // against 7.8 us, 24^3 equal, 32^3 13.9 against 8.9 us), and for P3 FP64 without
-  // whole cubes (37 x 41 x 35 hexes: 41.5 us, per hex 49.5 us).  Where 1 is the
-  // default and the mesh has enough patches (CGPatches), 1 runs cg_patch_kernel.
+  // Variant 0: the block form where it pays; cubes for P3 (two per SM at least: 28^3
+  // FP32 14.4, patches 14.9 us); P1 boxes with too little in a block go by hexes once
+  // there are many (2 x 200 x 400: FP64 hexes 12.2, patches 14.8 us; 48^3 9.4 / 11.7, but
+  // 37^3 7.1 / 7.5, 32^3 6.6 / 5.9); else 1, which is cg_patch_kernel if the mesh has
+  // enough patches (CGPatches), or a thread per cell.  P3 FP64 without whole cubes: 37 x
+  // 41 x 35 hexes 41.5 us by cells, per hex 49.5 us.
   int default_variant() const {
-    const bool cubes = cube_NB && n_blocks >= 2 * 148;
-    if (cfg.degree <= 2) return blocks.n_blocks >= 148 ? 3 : 1;
-    if (cubes || (sizeof(T) == 4 && blocks.n_blocks >= 148)) return 3;
+    if (blocks.pays(cfg.degree)) return 3;
+    if (cfg.degree == 3 && cube_NB && n_blocks >= 2 * 148) return 3;
+    if (cfg.degree == 1 && hex_H && n_hex >= 50000) return 2;
     return 1;
   }
 
@@ -688,7 +686,7 @@ class CGOperator final : public Operator {
     // measured fastest on B200 (FP64 P1 and P2: bank-scheduled with uniform steps;
     // FP32 and P3: contribution order)
     int sched = v >= 5 ? v - 5 : (sizeof(T) == 8 && cfg.degree <= 2 ? 1 : 0);
-    if (v == 3 && blocks.n_blocks && use_blocks()) {
+    if (v == 3 && use_blocks()) {
       blocks.launch(cfg.degree, x, d, d_constrained.n, d_constrained.p, s);
       return;
     }
@@ -746,7 +744,7 @@ class CGOperator final : public Operator {
   }
 
   const int32_t* device_dof_table() const override { return d_dofs.p; }
-  bool block_default() const override { return blocks.n_blocks && use_blocks() && default_variant() == 3; }
+  bool block_form() const override { return use_blocks() && blocks.n_blocks >= 148; }
   const BlockView* block_view() const override { return blocks.view.n_blocks ? &blocks.view : nullptr; }
 
   void element_matrices(void* out, cudaStream_t s) override {
@@ -828,12 +826,10 @@ class CGVectorOperator final : public Operator {
     d_constrained.upload(cl);
     blocks.build(mesh, cfg.degree, dofs.cell_dofs, dofs.constrained, geo);
     // P3 FP64 keeps the thread per cell: 44 x 40 x 36 hexes 130 us, by patches 137 to 160
-    if (!block_form() && (cfg.degree <= 2 || sizeof(T) == 4))
+    if (!blocks.pays(cfg.degree) && (cfg.degree <= 2 || sizeof(T) == 4))
       patches.build(cfg.degree, K, n_cells, dofs.cell_dofs, dofs.constrained);
   }
-  // P3 FP64: the block form is slower than a thread per cell (48^3 392 against 226 us)
-  bool block_form() const { return blocks.n_blocks >= 148 && (cfg.degree <= 2 || sizeof(T) == 4); }
-  bool block_default() const override { return block_form(); }
+  bool block_form() const override { return blocks.n_blocks >= 148; }
 
   void vmult(void* dst, const void* src, cudaStream_t s) override {
     vmult_phase(dst, src, 1, s);
@@ -847,7 +843,8 @@ class CGVectorOperator final : public Operator {
       SFEM_CUDA(cudaMemsetAsync(d, 0, sizeof(T) * m, s));
       return;
     }
-    if ((cfg.kernel_variant == 0 || cfg.kernel_variant == 3) && block_form()) {
+    const int v = cfg.kernel_variant;
+    if (blocks.n_blocks && (v == 3 || (v == 0 && blocks.pays(cfg.degree)))) {
       blocks.launch(cfg.degree, x, d, d_constrained.n, d_constrained.p, s);
       return;
     }

@@ -22,11 +22,47 @@ template <typename T, int NC>
 struct CGBlocks {
   DevBuf<int32_t> codes;
   DevBuf<uint8_t> upper;
-  BlockView view;  // also without the kernel (P3 FP64): the multigrid's transfers go by blocks
+  BlockView view;  // also without the kernel: the multigrid's transfers go by blocks
   DevBuf<int16_t> pos;
   DevBuf<T> geo;
-  int64_t n_blocks = 0;
-  int grid = 0;
+  int64_t n_blocks = 0, n_cells = 0;
+  int grid = 0, resident = 0;  // resident: CTAs that the device holds at once
+
+  // Whether the block form is the fastest one here.  A block costs the same however
+  // many of its 64 hexes are there (boxes thinner than four hexes, sides that four
+  // does not divide, a partition's cut), and a wave of blocks takes the time of one
+  // block; patches (cg_patch_kernel), cells and, for P1, hexes cost by the hex.  B200,
+  // us per vmult, block form / the fastest other one, hexes (per block):
+  //   P1, from 10,000 hexes (9000 (36) FP64 4.5 / 4.1; 10,600 (49) 4.4 / 4.4) and 34
+  //     (FP64) or 30 (FP32) per block: 160,000 (32) FP64 18.1 / 12.2, FP32 8.8 / 8.7;
+  //     56,700 (36) FP64 6.4 / 7.1; 160,000 (16) FP64 30.9 / 9.8, FP32 16.7 / 7.6.
+  //   P2 FP64, from 23,000: 21,952 (64) 8.2 / 7.3, 24,389 (48) 8.3 / 9.2; FP32 from
+  //     31,000: 27,000 (53) 7.3 / 6.9, 32,400 (48) 7.6 / 8.4; both from 42 per block,
+  //     38 where there are many: 50,000 (40) FP64 14.3 / 13.1, FP32 12.0 / 10.0;
+  //     38,400 (48) 10.4 / 10.8, 8.2 / 8.8; 150,000 (39) 37.6 / 39.0, 23.7 / 25.9;
+  //     160,000 (32) 47.3 / 38.2, 29.0 / 26.1.
+  //   P3 FP32 by waves w, about 3.5 + 12 w us against 0.5 us per 1000 hexes: 27,000
+  //     (one wave) 15.4 / 16.5, 35,937 (two) 26.5 / 18.1, 46,656 (two) 28.1 / 23.4,
+  //     53,095 (two) 26.7 / 25.5, 68,921 (three) 37.2 / 34.4, 110,592 (three) 38.9 / 43.9.
+  //   Three components, P1 from 10,000 and 24: 9000 (36) FP64 6.9 / 5.6, 25,000 (25) 8.5
+  //     / 9.7.  P2 FP64 from 42 per block and 18,000, or whole blocks: 17,576 (51) 15.5 /
+  //     14.2, 13,824 (64) 12.6 / 13.1, 20,800 (52) 15.6 / 16.8, 50,000 (40) 39.4 / 35.4.
+  //     P2 FP32 from 36 and 16,000: 15,625 (46) 11.6 / 10.8, 17,576 (51) 11.6 / 11.7,
+  //     40,000 (32) 22.0 / 20.5, 56,700 (36) 26.9 / 28.7.  P3 FP32 (no kernel): 46,656
+  //     (64) 79 / 70, 110,592 (64) 168 / 160, thin boxes 2 / 1.
+  bool pays(int p) const {
+    if (!n_blocks) return false;
+    const int64_t hexes = n_cells / 6;
+    const bool f64 = sizeof(T) == 8;
+    const double per = double(n_cells) / (6.0 * double(n_blocks));
+    if (NC == 3)
+      return p == 1 ? hexes >= 10000 && per >= 24
+             : f64  ? per >= 60 || (per >= 42 && hexes >= 18000)
+                    : per >= 36 && hexes >= 16000;
+    if (p == 1) return hexes >= 10000 && per >= (f64 ? 34 : 30);
+    if (p == 2) return hexes >= (f64 ? 23000 : 31000) && per >= (n_blocks >= 3000 ? 38 : 42);
+    return hexes >= 30000 * ((n_blocks + resident - 1) / resident) - 6000;
+  }
 
   // geo_soa: metric values [6][n_cells] in the operator's precision
   void build(const Mesh& mesh, int p, const std::vector<int32_t>& cell_dofs, const std::vector<uint8_t>& constrained,
@@ -40,7 +76,7 @@ struct CGBlocks {
     view.codes = codes.p;
     view.upper = upper.p;
     view.lattice = lattice;
-    if (p == 3 && sizeof(T) == 8) return;  // the slower kernel there (see CGOperator::use_blocks)
+    if (!has_kernel(p)) return;
     std::vector<T> g(size_t(36) * 64 * tb.n_blocks);
 #pragma omp parallel for schedule(static)
     for (int64_t b = 0; b < tb.n_blocks; ++b)
@@ -52,14 +88,19 @@ struct CGBlocks {
         }
     geo.upload(g);
     n_blocks = tb.n_blocks;
+    n_cells = mesh.n_cells;
     switch (p) {
       case 1: setup<1>(lattice); break;
       case 2: setup<2>(lattice); break;
       case 3:
-        if constexpr (sizeof(T) == 4) setup<3>(lattice);
+        if constexpr (has_kernel(3)) setup<3>(lattice);
         break;
     }
   }
+  // P3 FP64 (two resident CTAs of 64 threads): never the faster one (64^3 177 us, cubes
+  // 143 us; three components 48^3 392, a thread per cell 226 us), nor P3 FP32 with three
+  // components
+  static constexpr bool has_kernel(int p) { return p <= 2 || (sizeof(T) == 4 && NC == 1); }
 
   template <int P>
   static constexpr auto kernel() {
@@ -88,7 +129,8 @@ struct CGBlocks {
     SFEM_CUDA(cudaFuncSetAttribute(kernel<P>(), cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
     SFEM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel<P>(), 64, bytes));
     SFEM_REQUIRE(occ > 0, FEM_ERR_CUDA, "CG block kernel does not fit on an SM");
-    grid = int(std::min<int64_t>(n_blocks, int64_t(sms) * occ));
+    resident = sms * occ;
+    grid = int(std::min<int64_t>(n_blocks, resident));
   }
 
   template <int P>
@@ -101,7 +143,7 @@ struct CGBlocks {
       case 1: launch<1>(x, d, n_constrained, constrained, s); break;
       case 2: launch<2>(x, d, n_constrained, constrained, s); break;
       case 3:
-        if constexpr (sizeof(T) == 4) launch<3>(x, d, n_constrained, constrained, s);
+        if constexpr (has_kernel(3)) launch<3>(x, d, n_constrained, constrained, s);
         break;
     }
     SFEM_CUDA(cudaGetLastError());

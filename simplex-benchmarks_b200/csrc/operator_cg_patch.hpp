@@ -38,14 +38,22 @@ struct CGPatches {
   // (P2) and 0.39 (P3) distinct DoFs per cell and local DoF, rows of a box 0.41 for P3,
   // random order nearly one (24^3 hexes, patches / thread per cell: P2 FP64 10.3 / 9.4 us,
   // P3 FP64 23.4 / 16.2, P2 FP32 9.8 / 9.4, but P1 FP32 6.8 / 7.4, P3 FP32 14.8 / 19.3, three
-  // components P2 FP32 17.7 / 22).
+  // components P2 FP32 17.7 / 22).  P1 has to have half of its cells' DoFs free: constrained
+  // ones cost a thread per cell no gather and no atomic (1000 x 3 x 3 hexes, 44 % free: FP64
+  // 4.4 / 4.1, three components 5.9 / 5.5; 400 x 400 x 1, none: 11.1 / 10.4; 200 x 100 x 2,
+  // 50 %: 6.2 / 7.1; 1000 x 5 x 5, 64 %: 4.8 / 5.5).
   void build(int p, int K, int64_t nc, const std::vector<int32_t>& cell_dofs, const std::vector<uint8_t>& constrained) {
     if (nc == 0 || constrained.size() >= size_t(kPatchOwn)) return;
     const int BS = cells_of(p);
     const int64_t np = (nc + BS - 1) / BS;
     if (np < min_patches(p)) return;
     std::vector<int32_t> count(constrained.size(), 0);
-    for (int32_t g : cell_dofs) ++count[g];
+    int64_t free = 0;
+    for (int32_t g : cell_dofs) {
+      ++count[g];
+      free += !constrained[g];
+    }
+    if (p == 1 && double(free) < 0.47 * double(cell_dofs.size())) return;
     std::vector<uint32_t> sl(size_t(np) * (K / 2) * BS, 0);
     std::vector<std::vector<int32_t>> id(np);
     std::vector<std::vector<uint32_t>> en(np);
