@@ -447,10 +447,12 @@ int fem_batch_set_kernel_variant(fem_batch* batch, int32_t variant);
  * (median of `reps` launches after 2 warm-ups, on zero input), keeps the
  * fastest and returns it in *variant.  us[8] receives the median time per
  * variant 1..8 (0 = not a candidate; CG's approximate TF32 variant 4 is
- * never a candidate; CG's variant 3 is timed where it is the block form and
- * the default, its cube schedules as 5, 6 and 7).  With use_cache != 0 a choice recorded for
- * the same (kind, degree, precision, components, log2 cells, GPU name) is
- * applied without timing (*cached = 1).  fem_autotune_cache sets a file that
+ * never a candidate; CG's variant 3 is timed where it is the block form with
+ * 148 blocks or more, its cube schedules as 5, 6 and 7).  With use_cache != 0 a
+ * choice recorded for the same (kind, degree, precision, components, log2 cells,
+ * kernel forms that the mesh has, GPU name) is applied without timing
+ * (*cached = 1); records of a version whose variant numbers stood for other
+ * kernels are not used.  fem_autotune_cache sets a file that
  * keeps the choices across processes (JSON lines; NULL = memory only).
  * No counterpart in the reference (deal.II fixes its vectorisation at compile
  * time).  Synchronises with the device; allocates two vectors per problem. */

@@ -13,6 +13,10 @@ namespace sfem {
 
 namespace {
 
+// Raised when a variant number comes to stand for another kernel, so that choices
+// recorded before are not taken for the new one.
+constexpr int kKernelSet = 2;
+
 std::mutex g_mu;
 std::map<std::string, int> g_cache;
 std::string g_path;
@@ -50,11 +54,11 @@ std::vector<int> tune_candidates(const OpConfig& cfg) {
   return {1, 2, 3, 4, 5};
 }
 
-std::string tune_key(const OpConfig& cfg, int64_t cells) {
+std::string tune_key(const OpConfig& cfg, int64_t cells, const std::string& forms) {
   std::ostringstream os;
   const int lg = cells > 0 ? int(std::lround(std::log2(double(cells)))) : 0;
   os << "kind=" << cfg.kind << ",p=" << cfg.degree << ",prec=" << cfg.precision << ",nc=" << cfg.n_components
-     << ",log2cells=" << lg << ",gpu=" << device_name();
+     << ",log2cells=" << lg << ",set=" << kKernelSet << ",forms=" << forms << ",gpu=" << device_name();
   return os.str();
 }
 
@@ -109,7 +113,7 @@ TuneResult autotune(Operator& op, int reps, bool use_cache) {
   std::vector<int> cand = tune_candidates(op.cfg);
   if (op.block_form() && std::find(cand.begin(), cand.end(), 3) == cand.end()) cand.push_back(3);
   res.us.assign(8, 0.0);
-  const std::string key = tune_key(op.cfg, op.n_cells);
+  const std::string key = tune_key(op.cfg, op.n_cells, op.forms());
   if (use_cache) {
     const int v = tune_lookup(key);
     if (v > 0 && std::find(cand.begin(), cand.end(), v) != cand.end()) {

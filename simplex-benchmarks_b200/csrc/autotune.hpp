@@ -1,8 +1,9 @@
 // Kernel-shape autotuner: times every kernel variant (cells per CTA, thread
 // or warp roles per cell) of an operator or a multi-problem batch with CUDA
 // events and keeps the fastest.  Choices are cached per
-// (kind, degree, precision, components, log2 cells, GPU name) in memory and,
-// when a cache file is set, as JSON lines on disk.  No counterpart in the
+// (kind, degree, precision, components, log2 cells, kernel forms, GPU name) in
+// memory and, when a cache file is set, as JSON lines on disk.  The kernel forms
+// (Operator::forms) say which kernels the variant numbers stand for on a mesh.  No counterpart in the
 // reference (deal.II picks its vectorisation width at compile time).
 #pragma once
 #include <cuda_runtime.h>
@@ -17,8 +18,8 @@ namespace sfem {
 
 // candidate kernel variants of an operator configuration
 std::vector<int> tune_candidates(const OpConfig& cfg);
-// cache key of a configuration with `cells` cells in total
-std::string tune_key(const OpConfig& cfg, int64_t cells);
+// cache key of a configuration with `cells` cells in total and kernel forms `forms`
+std::string tune_key(const OpConfig& cfg, int64_t cells, const std::string& forms);
 // median device time (us) of `run` on `s` over `reps` launches after 2 warm-ups
 double time_launches(const std::function<void(cudaStream_t)>& run, int reps, cudaStream_t s);
 // cache access (thread-safe); lookup returns 0 when absent

@@ -4,6 +4,7 @@
 
 #include <cstdint>
 #include <memory>
+#include <string>
 #include <vector>
 
 #include "../../include/simplex_fem.h"
@@ -106,6 +107,8 @@ class Operator {
   // CG variant 3 is the block form here and has a block for every SM: the autotuner
   // times it too
   virtual bool block_form() const { return false; }
+  // which kernels the variants stand for on this mesh (part of the tuning key)
+  virtual std::string forms() const { return ""; }
   // Device scratch one vmult needs (DG: the published face traces; CG: none).
   virtual size_t scratch_bytes() const { return 0; }
   // vmult with the scratch supplied by the caller instead of the operator's own.

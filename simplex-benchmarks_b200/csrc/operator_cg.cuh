@@ -745,6 +745,11 @@ class CGOperator final : public Operator {
 
   const int32_t* device_dof_table() const override { return d_dofs.p; }
   bool block_form() const override { return use_blocks() && blocks.n_blocks >= 148; }
+  // default variant; 3 is the block form, cubes, hexes; 1 is the patch form
+  std::string forms() const override {
+    return std::to_string(default_variant()) + (use_blocks() ? "b" : "") + (cube_NB ? "c" : "") + (hex_H ? "h" : "") +
+           (patches.n_patches ? "p" : "");
+  }
   const BlockView* block_view() const override { return blocks.view.n_blocks ? &blocks.view : nullptr; }
 
   void element_matrices(void* out, cudaStream_t s) override {
@@ -830,6 +835,10 @@ class CGVectorOperator final : public Operator {
       patches.build(cfg.degree, K, n_cells, dofs.cell_dofs, dofs.constrained);
   }
   bool block_form() const override { return blocks.n_blocks >= 148; }
+  std::string forms() const override {
+    return std::string(blocks.pays(cfg.degree) ? "3" : "1") + (blocks.n_blocks ? "b" : "") +
+           (patches.n_patches ? "p" : "");
+  }
 
   void vmult(void* dst, const void* src, cudaStream_t s) override {
     vmult_phase(dst, src, 1, s);

@@ -212,6 +212,13 @@ class DGOperator final : public Operator {
     }
   }
 
+  // variant 1 in one launch or two
+  std::string forms() const override {
+    const DGProblem<T> pr = problem(nullptr, nullptr);
+    const bool one = cfg.degree <= 2 || (cfg.n_components == 1 ? fused3_pays<1>(&pr, 1) : fused3_pays<3>(&pr, 1));
+    return one ? "1" : "2";
+  }
+
   int status(bool clear) override {
     int v = 0;
     SFEM_CUDA(cudaMemcpy(&v, d_status.p, sizeof(int), cudaMemcpyDeviceToHost));
@@ -592,11 +599,16 @@ class DGBatchImpl final : public Batch {
     TuneResult res;
     res.us.assign(5, 0.0);
     int64_t cells = 0;
-    for (auto* o : ops) cells += o->n_cells;
-    const std::string key = "batch" + std::to_string(ops.size()) + "," + tune_key(cfg, cells);
+    std::string forms = "1";
+    for (auto* o : ops) {
+      cells += o->n_cells;
+      forms = std::max(forms, o->forms());  // one problem can send the launch to two
+    }
+    const std::vector<int> cand = tune_candidates(cfg);
+    const std::string key = "batch" + std::to_string(ops.size()) + "," + tune_key(cfg, cells, forms);
     if (use_cache) {
       const int v = tune_lookup(key);
-      if (v > 0) {
+      if (std::find(cand.begin(), cand.end(), v) != cand.end()) {
         cfg.kernel_variant = v;
         res.variant = v;
         res.cached = true;
@@ -620,7 +632,7 @@ class DGBatchImpl final : public Batch {
     const int keep = cfg.kernel_variant;
     double best = 1e300;
     try {
-      for (int v : tune_candidates(cfg)) {
+      for (int v : cand) {
         cfg.kernel_variant = v;
         const double us = time_launches([&](cudaStream_t st) { vmult(d.data(), x.data(), st); }, reps, s);
         res.us[v - 1] = us;
