@@ -647,6 +647,7 @@ class MultigridImpl final : public Multigrid {
       L.b.alloc(m);
       L.r.alloc(m);
       L.t.alloc(m);
+      clear_t(L, nullptr);
       L.d.alloc(m);
       L.op->inverse_diagonal(L.inv_diag.p, nullptr);
     }
