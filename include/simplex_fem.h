@@ -222,8 +222,10 @@ int fem_op_compute_diagonal(fem_op* op, void* diag, void* stream);
  * Running phase 1 then phase 2 equals fem_op_vmult. */
 int fem_op_vmult_phase(fem_op* op, void* dst, const void* src, int32_t phase, void* stream);
 /* Switch the kernel form of an existing operator (same meaning as
- * fem_op_params.kernel_variant); used by the autotuner.  No counterpart in
- * the reference (deal.II picks its vectorisation at compile time). */
+ * fem_op_params.kernel_variant); used by the autotuner.  A CG form's own tables
+ * are made when it is first asked for, here or at creation (device memory, and
+ * the calling thread waits).  No counterpart in the reference (deal.II picks its
+ * vectorisation at compile time). */
 int fem_op_set_kernel_variant(fem_op* op, int32_t variant);
 /* ---- assembled-matrix comparison -----------------------------------------
  * The reference compares its matrix-free vmult with a Trilinos sparse

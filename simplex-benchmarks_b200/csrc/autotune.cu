@@ -117,7 +117,7 @@ TuneResult autotune(Operator& op, int reps, bool use_cache) {
   if (use_cache) {
     const int v = tune_lookup(key);
     if (v > 0 && std::find(cand.begin(), cand.end(), v) != cand.end()) {
-      op.cfg.kernel_variant = v;
+      op.set_variant(v);
       res.variant = v;
       res.cached = true;
       return res;
@@ -132,7 +132,7 @@ TuneResult autotune(Operator& op, int reps, bool use_cache) {
   double best = 1e300;
   try {
     for (int v : cand) {
-      op.cfg.kernel_variant = v;
+      op.set_variant(v);
       const double us = time_launches([&](cudaStream_t st) { op.vmult(dst.p, src.p, st); }, reps, s);
       res.us[v - 1] = us;
       if (us < best) {

@@ -343,7 +343,7 @@ int fem_op_set_kernel_variant(fem_op* op, int32_t variant) {
                  "kernel_variant must be 0..8 (CG) or 0..5, 7, 9, 11 (DG, Helmholtz)");
     SFEM_REQUIRE((variant != 4 && variant != 8) || op->op->cfg.kind != FEM_CG || op->op->cfg.precision == FEM_FP32,
                  FEM_ERR_ARG, "CG kernel_variant 4 and 8 (TF32 tensor cores) are for FP32 operators");
-    op->op->cfg.kernel_variant = variant;
+    op->op->set_variant(variant);
   });
 }
 

@@ -1,14 +1,29 @@
 // Host helpers shared by the operator classes: space dimensions, launch grids
 // and the affine metric.
 #pragma once
+#include <cuda_runtime.h>
+
 #include <cmath>
 #include <cstdint>
 
+#include "common.hpp"
 #include "mesh.hpp"
 #include "ref_tables.h"
 
 namespace sfem {
 inline unsigned blocks_for(int64_t n, int bs) { return unsigned((n + bs - 1) / bs); }
+
+// Lets this thread allocate and copy while one of its streams is being captured.
+class RelaxedCapture {
+ public:
+  RelaxedCapture() { SFEM_CUDA(cudaThreadExchangeStreamCaptureMode(&mode_)); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+  RelaxedCapture(const RelaxedCapture&) = delete;
+  RelaxedCapture& operator=(const RelaxedCapture&) = delete;
+
+ private:
+  cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+};
 
 template <int P>
 inline int nnz_grad() {

@@ -48,6 +48,14 @@ struct DevBuf {
     }
   }
   void upload(const std::vector<T>& v) { upload(v.data(), v.size()); }
+  std::vector<T> download() const {
+    std::vector<T> v(n);
+    if (n) {
+      cudaError_t e = cudaMemcpy(v.data(), p, n * sizeof(T), cudaMemcpyDeviceToHost);
+      if (e != cudaSuccess) throw Error(FEM_ERR_CUDA, std::string("cudaMemcpy: ") + cudaGetErrorString(e));
+    }
+    return v;
+  }
   void release() {
     if (p) cudaFree(p);
     p = nullptr;
@@ -91,6 +99,9 @@ class Operator {
   std::vector<uint8_t> constrained;  // host mask [m]
   std::vector<double> support;       // host support points [m/NC][3]
 
+  // Switch the kernel form (fem_op_params.kernel_variant); a form's tables are made
+  // when it is first asked for.
+  virtual void set_variant(int v) { cfg.kernel_variant = v; }
   size_t elem_size() const { return cfg.precision == FEM_FP64 ? 8 : 4; }
   virtual void vmult(void* dst, const void* src, cudaStream_t s) = 0;
   // vmult onto a dst that is zero already where needs_zero() (callers that zero

@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <unordered_map>
 
 #include "kernels_cg.cuh"
@@ -27,8 +28,8 @@ class CGOperator final : public Operator {
   DevBuf<int32_t> d_dofs;        // [K][n_cells], -1 = constrained
   DevBuf<T> d_geo;               // [6][n_cells]
   DevBuf<int32_t> d_constrained; // constrained DoF list
-  // macro-element (hex) tables of cg_hex_kernel; empty when the mesh is not
-  // 6 consecutive Kuhn tets per hex with one common DoF pattern
+  // macro-element (hex) tables of cg_hex_kernel, made by make_hex_tables; hex_H = 0
+  // when the mesh is not 6 consecutive Kuhn tets per hex with one common DoF pattern
   DevBuf<int32_t> d_hdofs;       // [H][n_hex]
   DevBuf<T> d_hgeo;              // [36][n_hex]: metric of tet q at rows 6 q .. 6 q + 5
   HexMap hex_map{};
@@ -416,7 +417,8 @@ class CGOperator final : public Operator {
         d_status.p);
   }
 
-  void build_hex_tables(const Mesh& mesh, const CGDofs& dofs, const std::vector<T>& geo) {
+  // whether the mesh is 6 consecutive Kuhn tets per hex with one common DoF pattern
+  void find_hex_pattern(const Mesh& mesh, const CGDofs& dofs) {
     if (n_cells == 0 || n_cells % 6 != 0 || int64_t(mesh.cell_hex.size()) != n_cells) return;
     const int64_t nh = n_cells / 6;
     const int H = hex_dofs(cfg.degree);
@@ -441,7 +443,6 @@ class CGOperator final : public Operator {
     HexMap m0{};
     std::vector<int32_t> ord0;
     if (!local_map(0, m0.m, ord0)) return;
-    std::vector<int32_t> hd(size_t(H) * nh);
     bool ok = true;
 #pragma omp parallel
     {
@@ -453,24 +454,52 @@ class CGOperator final : public Operator {
         bool same = local_map(h, mm, ord);
         for (int q = 0; q < 6 && same; ++q)
           for (int i = 0; i < K; ++i) same = same && mm[q][i] == m0.m[q][i];
-        if (!same) {
-          ok = false;
-          continue;
-        }
-        for (int k = 0; k < H; ++k) hd[size_t(k) * nh + h] = dofs.constrained[ord[k]] ? -1 : ord[k];
+        if (!same) ok = false;
       }
     }
     if (!ok) return;
-    std::vector<T> hg(36 * size_t(nh));
-#pragma omp parallel for schedule(static)
-    for (int64_t h = 0; h < nh; ++h)
-      for (int q = 0; q < 6; ++q)
-        for (int k = 0; k < 6; ++k) hg[size_t(6 * q + k) * nh + h] = geo[size_t(k) * n_cells + 6 * h + q];
-    d_hgeo.upload(hg);
-    d_hdofs.upload(hd);
     hex_map = m0;
     n_hex = nh;
     hex_H = H;
+  }
+
+  // the hex form's DoF and metric tables, as large as the operator's own
+  void make_hex_tables() {
+    if (!hex_H || d_hdofs.n) return;
+    int first[64];  // tet and local DoF of every hex-local DoF
+    for (int q = 5; q >= 0; --q)
+      for (int i = K - 1; i >= 0; --i) first[hex_map.m[q][i]] = q * K + i;
+    const std::vector<T> geo = d_geo.download();
+    std::vector<int32_t> hd(size_t(hex_H) * n_hex);
+    std::vector<T> hg(36 * size_t(n_hex));
+#pragma omp parallel for schedule(static)
+    for (int64_t h = 0; h < n_hex; ++h) {
+      for (int k = 0; k < hex_H; ++k) {
+        const int32_t g = cell_dofs[size_t(K) * 6 * h + first[k]];
+        hd[size_t(k) * n_hex + h] = constrained[g] ? -1 : g;
+      }
+      for (int q = 0; q < 6; ++q)
+        for (int k = 0; k < 6; ++k) hg[size_t(6 * q + k) * n_hex + h] = geo[size_t(k) * n_cells + 6 * h + q];
+    }
+    d_hgeo.upload(hg);
+    d_hdofs.upload(hd);
+    SFEM_CUDA(cudaStreamSynchronize(nullptr));  // other streams do not wait for the copies
+  }
+
+  // the tables that only variant v's form reads
+  void make_tables(int v) {
+    if (v == 0) v = default_variant();
+    if (v == 3 && use_blocks()) blocks.make_metric(d_geo);
+    else if (v == 2 || ((v == 3 || (v >= 5 && v <= 7)) && !cube_NB)) make_hex_tables();
+  }
+  std::mutex tables_mutex;
+  void set_variant(int v) override {
+    {
+      std::lock_guard<std::mutex> lock(tables_mutex);
+      RelaxedCapture relaxed;
+      make_tables(v);
+    }
+    cfg.kernel_variant = v;
   }
 
   CGOperator(const Mesh& mesh, const OpConfig& c) : CGOperator(mesh, build_cg_dofs(mesh, c.degree), nullptr, c) {}
@@ -516,9 +545,9 @@ class CGOperator final : public Operator {
     for (int64_t i = 0; i < m; ++i)
       if (id_rows[i]) cl.push_back(int32_t(i));
     d_constrained.upload(cl);
-    build_hex_tables(mesh, dofs, geo);
+    find_hex_pattern(mesh, dofs);
     build_cube_tables(dofs);
-    blocks.build(mesh, cfg.degree, dofs.cell_dofs, dofs.constrained, geo);
+    blocks.build(mesh, cfg.degree, dofs.cell_dofs, dofs.constrained);
     if (default_variant() == 1) patches.build(cfg.degree, K, n_cells, dofs.cell_dofs, dofs.constrained);
     if (cfg.weak_bc) build_weak_boundary(mesh);
     d_status.alloc(1);
@@ -551,6 +580,7 @@ class CGOperator final : public Operator {
         case 3: setup_hex<3, 64>(); break;
       }
     }
+    make_tables(cfg.kernel_variant);
   }
 
   static constexpr int kHexBS = 64;
@@ -829,10 +859,23 @@ class CGVectorOperator final : public Operator {
     }
     d_geo.upload(geo);
     d_constrained.upload(cl);
-    blocks.build(mesh, cfg.degree, dofs.cell_dofs, dofs.constrained, geo);
+    blocks.build(mesh, cfg.degree, dofs.cell_dofs, dofs.constrained);
+    make_tables(cfg.kernel_variant);
     // P3 FP64 keeps the thread per cell: 44 x 40 x 36 hexes 130 us, by patches 137 to 160
     if (!blocks.pays(cfg.degree) && (cfg.degree <= 2 || sizeof(T) == 4))
       patches.build(cfg.degree, K, n_cells, dofs.cell_dofs, dofs.constrained);
+  }
+  void make_tables(int v) {
+    if (v == 3 || (v == 0 && blocks.pays(cfg.degree))) blocks.make_metric(d_geo);
+  }
+  std::mutex tables_mutex;
+  void set_variant(int v) override {
+    {
+      std::lock_guard<std::mutex> lock(tables_mutex);
+      RelaxedCapture relaxed;
+      make_tables(v);
+    }
+    cfg.kernel_variant = v;
   }
   bool block_form() const override { return blocks.n_blocks >= 148; }
   std::string forms() const override {

@@ -64,11 +64,12 @@ struct CGBlocks {
     return hexes >= 30000 * ((n_blocks + resident - 1) / resident) - 6000;
   }
 
-  // geo_soa: metric values [6][n_cells] in the operator's precision
-  void build(const Mesh& mesh, int p, const std::vector<int32_t>& cell_dofs, const std::vector<uint8_t>& constrained,
-             const std::vector<T>& geo_soa) {
+  std::vector<int32_t> cell;  // of every block's hexes' tets, until the metric by blocks is made
+
+  // everything but the metric by blocks
+  void build(const Mesh& mesh, int p, const std::vector<int32_t>& cell_dofs, const std::vector<uint8_t>& constrained) {
     const std::vector<int32_t> lattice = p == 1 ? slots<1>() : p == 2 ? slots<2>() : slots<3>();
-    const CGBlockTables tb = build_cg_block_tables(mesh, p, cell_dofs, constrained, lattice);
+    CGBlockTables tb = build_cg_block_tables(mesh, p, cell_dofs, constrained, lattice);
     if (!tb.n_blocks) return;
     codes.upload(tb.codes);
     upper.upload(tb.upper);
@@ -77,18 +78,9 @@ struct CGBlocks {
     view.upper = upper.p;
     view.lattice = lattice;
     if (!has_kernel(p)) return;
-    std::vector<T> g(size_t(36) * 64 * tb.n_blocks);
-#pragma omp parallel for schedule(static)
-    for (int64_t b = 0; b < tb.n_blocks; ++b)
-      for (int q = 0; q < 6; ++q)
-        for (int t = 0; t < 64; ++t) {
-          const int64_t c = tb.cell[384 * b + 64 * q + t];
-          for (int k = 0; k < 6; ++k)
-            g[(36 * size_t(b) + 6 * q + k) * 64 + t] = c >= 0 ? geo_soa[size_t(k) * mesh.n_cells + c] : T(0);
-        }
-    geo.upload(g);
     n_blocks = tb.n_blocks;
     n_cells = mesh.n_cells;
+    cell = std::move(tb.cell);
     switch (p) {
       case 1: setup<1>(lattice); break;
       case 2: setup<2>(lattice); break;
@@ -96,6 +88,23 @@ struct CGBlocks {
         if constexpr (has_kernel(3)) setup<3>(lattice);
         break;
     }
+  }
+  // the metric by blocks, as large as the operator's own: made where the form runs
+  void make_metric(const DevBuf<T>& d_geo) {
+    if (!n_blocks || geo.n) return;
+    const std::vector<T> soa = d_geo.download();  // [6][n_cells]
+    std::vector<T> g(size_t(36) * 64 * n_blocks);
+#pragma omp parallel for schedule(static)
+    for (int64_t b = 0; b < n_blocks; ++b)
+      for (int q = 0; q < 6; ++q)
+        for (int t = 0; t < 64; ++t) {
+          const int64_t c = cell[384 * b + 64 * q + t];
+          for (int k = 0; k < 6; ++k)
+            g[(36 * size_t(b) + 6 * q + k) * 64 + t] = c >= 0 ? soa[size_t(k) * n_cells + c] : T(0);
+        }
+    geo.upload(g);
+    SFEM_CUDA(cudaStreamSynchronize(nullptr));  // other streams do not wait for the copy
+    cell = {};
   }
   // P3 FP64 (two resident CTAs of 64 threads): never the faster one (64^3 177 us, cubes
   // 143 us; three components 48^3 392, a thread per cell 226 us), nor P3 FP32 with three
