@@ -3,8 +3,10 @@
 // by operator_dg_f64.cu and operator_dg_f32.cu.
 #pragma once
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 
 #include "autotune.hpp"
 #include "kernels_dg.cuh"
@@ -24,6 +26,7 @@ namespace {
 template <typename T>
 class DGOperator final : public Operator {
  public:
+  // for the two-launch forms and the diagonal (made by need_geometry)
   DevBuf<T> d_geo;      // [6 + 4 + (mass?1:0)][n_cells]
   DevBuf<int32_t> d_nb; // [4][n_cells]
   DevBuf<int8_t> d_nbf; // [4][n_cells]
@@ -35,7 +38,8 @@ class DGOperator final : public Operator {
   DevBuf<OuterFace<T>> d_outer;
   int n_outer = 0;
   DevBuf<T> d_Q;        // published face normal derivatives: [n_cells][4][NC][NFQ], or block-major
-                        // (scalar problems, 1-thread-per-cell forms), for whole 128-cell blocks
+                        // (scalar problems, 1-thread-per-cell forms), for whole 128-cell blocks; made by
+                        // need_traces
   DevBuf<int> d_status; // timeouts of the bounded waits in the bulk-copy trace pass
   bool has_mass = false;
 
@@ -102,20 +106,10 @@ class DGOperator final : public Operator {
         }
         geo[size_t(6 + f) * n_cells + cc] = T(sigma * area[4 * cc + f]);
       }
-    d_geo.upload(geo);
-    std::vector<int32_t> nb(4 * size_t(n_cells));
-    std::vector<int8_t> nbf(4 * size_t(n_cells));
-    for (int64_t cc = 0; cc < n_cells; ++cc)
-      for (int f = 0; f < 4; ++f) {
-        nb[size_t(f) * n_cells + cc] = std::max(mesh.nb[4 * cc + f], -1);
-        nbf[size_t(f) * n_cells + cc] = mesh.nbf[4 * cc + f] < 0 ? 0 : mesh.nbf[4 * cc + f];
-      }
-    d_nb.upload(nb);
-    d_nbf.upload(nbf);
     build_fused(mesh, geo);
-    d_Q.alloc(size_t((n_cells + kQB - 1) / kQB * kQB) * 4 * cfg.n_components * nfq_of(p));
     d_status.alloc(1);
     SFEM_CUDA(cudaMemset(d_status.p, 0, sizeof(int)));
+    set_variant(cfg.kernel_variant);
   }
 
   // cells of a block of the single-launch form
@@ -126,11 +120,26 @@ class DGOperator final : public Operator {
 
   // Geometry, outer neighbours and (P3) outer faces by blocks of cells: FusedShape
   // (P1, P2) and Fused3Shape (P3)
+  struct FusedLayout {
+    bool p3;
+    int64_t BS;
+    int NG;        // values per cell
+    size_t bytes;  // of a block: the values, then four face codes per cell
+  };
+  FusedLayout fused_layout() const {
+    FusedLayout L;
+    L.p3 = cfg.degree == 3;
+    L.BS = fused_block();
+    L.NG = (L.p3 ? 10 : 22) + (has_mass ? 1 : 0);
+    L.bytes = size_t(L.NG) * L.BS * sizeof(T) + 4 * L.BS * (L.p3 ? sizeof(uint32_t) : sizeof(uint16_t));
+    return L;
+  }
   void build_fused(const Mesh& mesh, const std::vector<T>& geo) {
-    const int64_t BS = fused_block(), nblk = (n_cells + BS - 1) / BS;
-    const bool p3 = cfg.degree == 3;
-    const int NG = (p3 ? 10 : 22) + (has_mass ? 1 : 0);
-    const size_t block_bytes = size_t(NG) * BS * sizeof(T) + 4 * BS * (p3 ? sizeof(uint32_t) : sizeof(uint16_t));
+    const FusedLayout L = fused_layout();
+    const int64_t BS = L.BS, nblk = (n_cells + BS - 1) / BS;
+    const bool p3 = L.p3;
+    const int NG = L.NG;
+    const size_t block_bytes = L.bytes;
     std::vector<unsigned char> fg(block_bytes * nblk, 0);
     std::vector<std::vector<int32_t>> outer(nblk);
     std::vector<std::vector<OuterFace<T>>> faces(p3 ? nblk : 0);
@@ -212,11 +221,78 @@ class DGOperator final : public Operator {
     }
   }
 
+  // Geometry by cells and trace buffer, which the single-launch forms do not read
+  // (Helmholtz P2 FP64: 108 and 288 of 607 bytes a cell): made when a two-launch form or
+  // the diagonal is first asked for.
+  std::mutex tables_mutex;
+  std::atomic<bool> have_geometry{false}, have_traces{false};
+
+  void need_geometry() {
+    if (have_geometry.load(std::memory_order_acquire)) return;
+    std::lock_guard<std::mutex> lock(tables_mutex);
+    if (have_geometry.load(std::memory_order_relaxed)) return;
+    RelaxedCapture relaxed;
+    const FusedLayout L = fused_layout();
+    const std::vector<unsigned char> fg = d_fgeo.download();
+    const std::vector<int32_t> begin = d_ext_begin.download(), ext = d_ext.download();
+    const size_t n = size_t(n_cells);
+    std::vector<T> geo((has_mass ? 11 : 10) * n);
+    std::vector<int32_t> nb(4 * n);
+    std::vector<int8_t> nbf(4 * n);
+#pragma omp parallel for schedule(static)
+    for (int64_t c = 0; c < n_cells; ++c) {
+      const int64_t b = c / L.BS, at = c % L.BS;
+      const T* g = reinterpret_cast<const T*>(fg.data() + b * L.bytes);
+      for (int k = 0; k < 10; ++k) geo[k * n + c] = g[k * L.BS + at];
+      if (has_mass) geo[10 * n + c] = g[(L.NG - 1) * L.BS + at];
+      const void* codes = g + L.NG * L.BS;
+      for (int f = 0; f < 4; ++f) {
+        const uint32_t code3 = L.p3 ? static_cast<const uint32_t*>(codes)[f * L.BS + at] : 0;
+        const uint16_t code = L.p3 ? uint16_t(0) : static_cast<const uint16_t*>(codes)[f * L.BS + at];
+        const bool boundary = L.p3 ? code3 == kBoundary3 : code == kBoundary;
+        const int64_t row = L.p3 ? code3 & 0x3FFFu : code >> 2;
+        nb[f * n + c] = boundary ? -1 : row < L.BS ? int32_t(b * L.BS + row) : ext[begin[b] + row - L.BS];
+        nbf[f * n + c] = boundary ? 0 : int8_t(L.p3 ? code3 >> 14 & 3u : code & 3u);
+      }
+    }
+    d_geo.upload(geo);
+    d_nb.upload(nb);
+    d_nbf.upload(nbf);
+    SFEM_CUDA(cudaStreamSynchronize(nullptr));  // other streams do not wait for the copies
+    have_geometry.store(true, std::memory_order_release);
+  }
+  size_t trace_values() const {
+    return size_t((n_cells + kQB - 1) / kQB * kQB) * 4 * cfg.n_components * nfq_of(cfg.degree);
+  }
+  void need_traces() {
+    if (have_traces.load(std::memory_order_acquire)) return;
+    std::lock_guard<std::mutex> lock(tables_mutex);
+    if (have_traces.load(std::memory_order_relaxed)) return;
+    RelaxedCapture relaxed;
+    d_Q.alloc(trace_values());
+    have_traces.store(true, std::memory_order_release);
+  }
+  // vmult with variant v takes one launch
+  bool one_launch(int v) const {
+    const DGProblem<T> pr = problem(nullptr, nullptr);
+    return one_launch(cfg, &pr, 1, v);
+  }
+  static bool one_launch(const OpConfig& cfg, const DGProblem<T>* probs, int n, int v) {
+    if (v == 0) v = default_variant(cfg.degree, cfg.n_components, 0);
+    if (v != 1) return false;
+    return cfg.degree <= 2 || (cfg.n_components == 1 ? fused3_pays<1>(probs, n) : fused3_pays<3>(probs, n));
+  }
+  void set_variant(int v) override {
+    if (!one_launch(v)) {
+      need_geometry();
+      need_traces();
+    }
+    cfg.kernel_variant = v;
+  }
+
   // variant 1 in one launch or two
   std::string forms() const override {
-    const DGProblem<T> pr = problem(nullptr, nullptr);
-    const bool one = cfg.degree <= 2 || (cfg.n_components == 1 ? fused3_pays<1>(&pr, 1) : fused3_pays<3>(&pr, 1));
-    return one ? "1" : "2";
+    return one_launch(1) ? "1" : "2";
   }
 
   int status(bool clear) override {
@@ -251,11 +327,13 @@ class DGOperator final : public Operator {
   }
 
   void vmult_phase(void* dst, const void* src, int phase, cudaStream_t s) override {
+    need_geometry();
+    need_traces();
     const DGProblem<T> pr = problem(src, dst);
     launch_dg(cfg, &pr, 1, s, phase, d_status.p);
   }
 
-  size_t scratch_bytes() const override { return d_Q.n * sizeof(T); }
+  size_t scratch_bytes() const override { return trace_values() * sizeof(T); }
 
   void vmult_with_scratch(void* dst, const void* src, void* scratch, size_t bytes, cudaStream_t s) override {
     SFEM_REQUIRE(bytes >= scratch_bytes(), FEM_ERR_ARG, "vmult: scratch too small");
@@ -265,6 +343,7 @@ class DGOperator final : public Operator {
   }
 
   void diagonal(void* diag, cudaStream_t s) override {
+    need_geometry();
     const DGProblem<T> pr = problem(nullptr, diag);
     launch_dg(cfg, &pr, 1, s, 3, d_status.p);
   }
@@ -580,6 +659,7 @@ class DGBatchImpl final : public Batch {
       q_of.push_back(repeat);
       ops.push_back(d);
     }
+    set_variant(cfg.kernel_variant);
   }
   void vmult(void* const* dst, const void* const* src, cudaStream_t s) override {
     DGProblem<T> probs[kMaxBatch];
@@ -593,6 +673,13 @@ class DGBatchImpl final : public Batch {
   void set_variant(int v) override {
     SFEM_REQUIRE(v >= 0 && v <= 11 && v != 6 && v != 8 && v != 10, FEM_ERR_ARG,
                  "batch: kernel variant must be 0..5, 7, 9 or 11");
+    DGProblem<T> probs[kMaxBatch];
+    for (size_t i = 0; i < ops.size(); ++i) probs[i] = ops[i]->problem(nullptr, nullptr);
+    if (!DGOperator<T>::one_launch(cfg, probs, int(ops.size()), v))
+      for (auto* o : ops) {
+        o->need_geometry();
+        o->need_traces();
+      }
     cfg.kernel_variant = v;
   }
   TuneResult tune(int reps, bool use_cache) override {
@@ -609,7 +696,7 @@ class DGBatchImpl final : public Batch {
     if (use_cache) {
       const int v = tune_lookup(key);
       if (std::find(cand.begin(), cand.end(), v) != cand.end()) {
-        cfg.kernel_variant = v;
+        set_variant(v);
         res.variant = v;
         res.cached = true;
         return res;
@@ -633,7 +720,7 @@ class DGBatchImpl final : public Batch {
     double best = 1e300;
     try {
       for (int v : cand) {
-        cfg.kernel_variant = v;
+        set_variant(v);
         const double us = time_launches([&](cudaStream_t st) { vmult(d.data(), x.data(), st); }, reps, s);
         res.us[v - 1] = us;
         if (us < best) {
