@@ -239,7 +239,8 @@ int fem_op_set_kernel_variant(fem_op* op, int32_t variant);
 int fem_op_element_matrices(fem_op* op, void* mats, void* stream);
 int fem_csr_spmv(int64_t n_rows, const int64_t* row_ptr, const int32_t* col, const void* val, const void* x,
                  void* y, int32_t precision, void* stream);
-/* Algorithmic work of one vmult: flops and bytes of the fused kernels. */
+/* Algorithmic work of one vmult: flops of the fused kernels; bytes of src and dst
+ * and of the tables that the operator's current kernel form reads, each once. */
 int fem_op_work(const fem_op* op, double* flops, double* bytes);
 /* Device-side status of the operator's kernels since the last call, then
  * cleared: bit 0 = a kernel gave up on a bounded wait (a tensor-core CG

@@ -134,8 +134,8 @@ class Operator {
   // device-side status bits of the operator's kernels since the last call
   // (bit 0: a tensor-core kernel gave up on a bounded wait); clear resets them
   virtual int status(bool clear) { return 0; }
-  // flops of the fused kernels and algorithmic bytes (src+dst once, index and
-  // geometry data once) of one vmult
+  // flops of the fused kernels and algorithmic bytes (src and dst once, the index and
+  // geometry tables of the current kernel form once) of one vmult
   virtual void work(double& flops, double& bytes) const = 0;
   // dst = (f, v_i) for the load described by `rhs` (CG: 0 on constrained DoFs)
   virtual void rhs(const struct RhsDesc& rhs, void* dst, cudaStream_t s);

@@ -797,8 +797,18 @@ class CGOperator final : public Operator {
     const int p = cfg.degree, kq = kq_of(p);
     const double per_cell = 2.0 * (2 * nnz_grad_rt(p) + 9 * kq + 3 * kq * kq);
     flops = per_cell * double(n_cells);
-    const double s = double(sizeof(T));
-    bytes = 2 * s * double(m) + 4.0 * K * double(n_cells) + 6 * s * double(n_cells);
+    bytes = 2.0 * sizeof(T) * double(m) + double(table_bytes());
+  }
+  // index and metric tables that the current form reads
+  size_t table_bytes() const {
+    const size_t metric = d_geo.n * sizeof(T);
+    int v = cfg.kernel_variant == 0 ? default_variant() : cfg.kernel_variant;
+    if (v == 3 && use_blocks()) return blocks.table_bytes();
+    if ((v == 3 || v >= 5) && cube_NB) return metric + d_bdof.n * sizeof(int32_t);
+    if (v == 2 || v == 3 || (v >= 5 && v <= 7))
+      if (hex_H) return metric + size_t(hex_H) * n_hex * sizeof(int32_t);
+    if (v == 1 && patches.n_patches) return metric + patches.table_bytes();
+    return metric + d_dofs.n * sizeof(int32_t);
   }
 };
 
@@ -940,8 +950,12 @@ class CGVectorOperator final : public Operator {
   void work(double& flops, double& bytes) const override {
     const int p = cfg.degree, kq = kq_of(p);
     flops = NC * 2.0 * (2 * nnz_grad_rt(p) + 9 * kq + 3 * kq * kq) * double(n_cells);
-    const double sz = double(sizeof(T));
-    bytes = 2 * sz * double(m) + 4.0 * K * double(n_cells) + 6 * sz * double(n_cells);
+    const int v = cfg.kernel_variant;
+    const bool by_blocks = blocks.n_blocks && (v == 3 || (v == 0 && blocks.pays(p)));
+    const size_t tables = by_blocks ? blocks.table_bytes()
+                                    : d_geo.n * sizeof(T) + (patches.n_patches ? patches.table_bytes()
+                                                                               : d_dofs.n * sizeof(int32_t));
+    bytes = 2.0 * sizeof(T) * double(m) + double(tables);
   }
 };
 

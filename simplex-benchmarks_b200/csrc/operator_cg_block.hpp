@@ -106,6 +106,8 @@ struct CGBlocks {
     SFEM_CUDA(cudaStreamSynchronize(nullptr));  // other streams do not wait for the copy
     cell = {};
   }
+  // codes and metric that a product reads
+  size_t table_bytes() const { return codes.n * sizeof(int32_t) + size_t(36) * 64 * n_blocks * sizeof(T); }
   // P3 FP64 (two resident CTAs of 64 threads): never the faster one (64^3 177 us, cubes
   // 143 us; three components 48^3 392, a thread per cell 226 us), nor P3 FP32 with three
   // components

@@ -15,7 +15,9 @@ struct CGPatches {
   DevBuf<uint32_t> slots, entries;
   DevBuf<int32_t> ids, n_ids, ent_begin;
   PatchTables tb{};
-  int64_t n_patches = 0, n_cells = 0;
+  int64_t n_patches = 0, n_cells = 0, n_distinct = 0;
+  // slots, distinct DoFs and lists that a product reads
+  size_t table_bytes() const { return 4 * (slots.n + entries.n + size_t(n_distinct)); }
 
   static int cells_of(int p) {
     return p == 1 ? cg_patch_cells<1, NC>() : p == 2 ? cg_patch_cells<2, NC>() : cg_patch_cells<3, NC>();
@@ -136,6 +138,7 @@ struct CGPatches {
     tb.entries = entries.p;
     tb.ent_begin = ent_begin.p;
     n_cells = nc;
+    n_distinct = total;
     n_patches = np;
   }
 
