@@ -647,15 +647,17 @@ def write_kernels(data, path):
                 rows.append(lat.index(tuple(b)))
             assert rows[:NF] == d["FN"][f]
             d["SIDE"].append(rows)
-        # derivatives along v_w - opposite vertex at the P_{p-1} face nodes (face 3)
-        side = d["SIDE"][3]
-        along = []
-        for w in range(3):
-            for m in d["FNQ"][3]:
-                row = [(d["D"][w - 1][m][i] if w else Fr(0)) - d["D"][2][m][i] for i in range(K)]
-                along.append([row[side[i]] for i in range(K)])
-        product_fn(f"g[w*{NFQ}+m] = derivative along v_w - o at face node m, from a cell's values in side order",
-                   f"sideGrad_P{p}(const T* s, T* g)", along, lambda r: f"g[{r}]", lambda c: f"s[{c}]")
+        # derivatives along v_w - opposite vertex at the P_{p-1} face nodes (face 3), for
+        # the one-launch DG P3 form
+        if p == 3:
+            side = d["SIDE"][3]
+            along = []
+            for w in range(3):
+                for m in d["FNQ"][3]:
+                    row = [(d["D"][w - 1][m][i] if w else Fr(0)) - d["D"][2][m][i] for i in range(K)]
+                    along.append([row[side[i]] for i in range(K)])
+            product_fn(f"g[w*{NFQ}+m] = derivative along v_w - o at face node m, from a cell's values in side order",
+                       f"sideGrad_P{p}(const T* s, T* g)", along, lambda r: f"g[{r}]", lambda c: f"s[{c}]")
         # the same three row by row, for the CG kernels that run out of registers
         # before they run out of arithmetic (see cg_local_apply)
         body = []
@@ -665,9 +667,6 @@ def write_kernels(data, path):
         body = []
         emit_matvec(body, [list(c) for c in zip(*DD)], K, 3 * KQ, lambda r: f"y[{r}]", lambda c: f"h[{c}]", True)
         fn("gradT, row by row", f"gradTRows_P{p}(const T (&h)[{3*KQ}], T (&y)[{K}])", body)
-        body = []
-        emit_matvec(body, [list(c) for c in zip(*DD)], K, 3 * KQ, lambda r: f"y({r})", lambda c: f"h[{c}]", True)
-        fn("gradTInto, row by row", f"gradTRowsInto_P{p}(const T (&h)[{3*KQ}], F&& y)", body)
         body = []
         emit_matvec(body, d["MQ"], KQ, KQ, lambda r: f"o[{r}]", lambda c: f"w[{c}]", False)
         fn("massQ, row by row", f"massQRows_P{p}(const T* w, T* o)", body)
@@ -766,7 +765,6 @@ def write_kernels(data, path):
         L.append(f"  template <class T> static __device__ __forceinline__ void gradRows(const T (&u)[{K}], T (&g)[{3*KQ}]) {{ gradRows_P{p}(u, g); }}")
         L.append(f"  template <class T> static __device__ __forceinline__ void gradTRows(const T (&h)[{3*KQ}], T (&y)[{K}]) {{ gradTRows_P{p}(h, y); }}")
         L.append(f"  template <class T, class F> static __device__ __forceinline__ void gradTInto(const T (&h)[{3*KQ}], F&& y) {{ gradTInto_P{p}(h, y); }}")
-        L.append(f"  template <class T, class F> static __device__ __forceinline__ void gradTRowsInto(const T (&h)[{3*KQ}], F&& y) {{ gradTRowsInto_P{p}(h, y); }}")
         L.append(f"  template <class T> static __device__ __forceinline__ void massQRows(const T* w, T* o) {{ massQRows_P{p}(w, o); }}")
         L.append(f"  template <class T, class F> static __device__ __forceinline__ void faceFlux(const T* a, F&& o) {{ faceFlux_P{p}(a, o); }}")
         L.append(f"  template <class T> static __device__ __forceinline__ void faceTest(const T* t, T* o) {{ faceTest_P{p}(t, o); }}")
@@ -784,9 +782,10 @@ def write_kernels(data, path):
         L.append(f"  static __host__ __device__ __forceinline__ constexpr int faceq_pos(int f, int m) {{ return faceq_pos_P{p}(f, m); }}")
         cases = " ".join(f"case {f*NF+i}: return {d['FN'][f][i]};" for f in range(4) for i in range(NF))
         L.append(f"  static __host__ __device__ __forceinline__ constexpr int fn(int f, int i) {{ switch (f * {NF} + i) {{ {cases} }} return 0; }}")
-        L.append(f"  template <class T> static __device__ __forceinline__ void sideGrad(const T* s, T* g) {{ sideGrad_P{p}(s, g); }}")
-        cases = " ".join(f"case {f*K+i}: return {d['SIDE'][f][i]};" for f in range(4) for i in range(K))
-        L.append(f"  static __host__ __device__ __forceinline__ constexpr int side(int f, int i) {{ switch (f * {K} + i) {{ {cases} }} return 0; }}")
+        if p == 3:
+            L.append(f"  template <class T> static __device__ __forceinline__ void sideGrad(const T* s, T* g) {{ sideGrad_P{p}(s, g); }}")
+            cases = " ".join(f"case {f*K+i}: return {d['SIDE'][f][i]};" for f in range(4) for i in range(K))
+            L.append(f"  static __host__ __device__ __forceinline__ constexpr int side(int f, int i) {{ switch (f * {K} + i) {{ {cases} }} return 0; }}")
         # Kuhn hex: lattice offset (x, y, z in 0..p) of node i of tet q.  Tet q walks
         # the hex edges in axis order KUHN[q], which is also the order of its
         # (ascending) vertices.
