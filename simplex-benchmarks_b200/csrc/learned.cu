@@ -79,10 +79,15 @@ LearnedSmoother::LearnedSmoother(uint64_t seed) {
   v_.alloc(NP);
   g_.alloc(NP);
   sums_.alloc(NP + 1);
+  SFEM_CUDA(cudaMallocHost(&host_loss_, sizeof(double)));
   wb_.alloc(NP);
   status_.alloc(1);
   SFEM_CUDA(cudaMemset(status_.p, 0, sizeof(int)));
   set_weights(w);
+}
+
+LearnedSmoother::~LearnedSmoother() {
+  if (host_loss_) cudaFreeHost(host_loss_);
 }
 
 std::vector<float> LearnedSmoother::host_weights() const {
@@ -170,7 +175,7 @@ GradPlan mlp_grad_plan(int n, int sms) {
 }  // namespace
 
 void LearnedSmoother::launch_gradient(const float* X, const float* Y, int n, float* grad, bool accumulate_loss,
-                                      cudaStream_t s) {
+                                      double* loss, cudaStream_t s) {
   static std::atomic<uint64_t> configured{0};
   int dev = 0, sms = 0;
   SFEM_CUDA(cudaGetDevice(&dev));
@@ -190,7 +195,7 @@ void LearnedSmoother::launch_gradient(const float* X, const float* Y, int n, flo
   else
     mlp_grad_kernel<2><<<p.grid, mlpg::THREADS, mlpg::Shape<2>::BYTES, s>>>(n, X, Y, wb_.p, sums_.p, sums_.p + NP, inv);
   SFEM_CUDA(cudaGetLastError());
-  launch_pdl(mlp_grad_round_kernel, (NP + 255) / 256, 256, 0, s, sums_.p, grad);
+  launch_pdl(mlp_grad_round_kernel, NP / 256 + 1, 256, 0, s, sums_.p, grad, loss);
 }
 
 double LearnedSmoother::read_loss(cudaStream_t s) {
@@ -202,8 +207,9 @@ double LearnedSmoother::read_loss(cudaStream_t s) {
 
 double LearnedSmoother::gradient(const float* X, const float* Y, int n, float* grad, cudaStream_t s) {
   std::lock_guard<std::mutex> lock(sums_mutex_);  // until the loss is read: the sums are the handle's
-  launch_gradient(X, Y, n, grad, false, s);
-  return read_loss(s);
+  launch_gradient(X, Y, n, grad, false, host_loss_, s);
+  SFEM_CUDA(cudaStreamSynchronize(s));
+  return *host_loss_;
 }
 
 void LearnedSmoother::forward(const float* X, float* O, int n, cudaStream_t s) {
@@ -248,7 +254,7 @@ TrainStats LearnedSmoother::train(const float* X, const float* Y, int n, int epo
     for (int off = 0; off + batch <= n || (off < n && nb == 0); off += batch) {
       const int cnt = std::min(batch, n - off);
       // the epoch's losses add up on the device, read back once per epoch
-      launch_gradient(Xp.p + int64_t(off) * D::NIN, Yp.p + int64_t(off) * D::NOUT, cnt, g_.p, nb > 0, s);
+      launch_gradient(Xp.p + int64_t(off) * D::NIN, Yp.p + int64_t(off) * D::NOUT, cnt, g_.p, nb > 0, nullptr, s);
       ++adam_t_;
       const float c1 = 1.0f / (1.0f - std::pow(b1, float(adam_t_)));
       const float c2 = 1.0f / (1.0f - std::pow(b2, float(adam_t_)));

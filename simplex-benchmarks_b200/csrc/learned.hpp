@@ -43,6 +43,7 @@ struct TrainStats {
 class LearnedSmoother {
  public:
   explicit LearnedSmoother(uint64_t seed);
+  ~LearnedSmoother();
   static constexpr int NP = MLPDims::NPARAM;
   std::vector<float> host_weights() const;
   void set_weights(const std::vector<float>& w);
@@ -73,12 +74,15 @@ class LearnedSmoother {
   };
   Bound& bind(const Operator& op);
   void round_weights(cudaStream_t s);
-  // gradient of the batch into grad and its loss (mean) into sums_[NP], or added to it; no
-  // synchronisation, the caller holds sums_mutex_ until read_loss
-  void launch_gradient(const float* X, const float* Y, int n, float* grad, bool accumulate_loss, cudaStream_t s);
+  // gradient of the batch into grad and its loss (mean) into sums_[NP], or added to it, and
+  // to *loss (pinned) unless that is null; no synchronisation, the caller holds sums_mutex_
+  // until it has read the loss
+  void launch_gradient(const float* X, const float* Y, int n, float* grad, bool accumulate_loss, double* loss,
+                       cudaStream_t s);
   double read_loss(cudaStream_t s);
   DevBuf<float> w_, m_, v_, g_;
   DevBuf<double> sums_;  // [NP] gradient sums, loss
+  double* host_loss_ = nullptr;  // pinned
   std::mutex sums_mutex_;
   DevBuf<__nv_bfloat16> wb_;
   DevBuf<int> status_;

@@ -12,7 +12,7 @@
 // over all tiles of the CTA and leave once, as coalesced atomic additions in FP64
 // that a second small launch rounds.  Added in FP32, one CTA's sums after another onto
 // the same total (128 CTAs for 2048 samples), the gradient's error against 64 bits is
-// 1.6e-7 at 2048 and 2.2e-7 at 8192 samples; so it is 3e-8 at both, for 1.3 us of a
+// 1.6e-7 at 2048 and 2.2e-7 at 8192 samples; so it is 3e-8 at both, for 2 us of a
 // call.  Eight or four CTAs of a cluster adding pairwise before an FP32 addition leave
 // 6e-8 and 8e-8, but 16 clusters of eight or more than 33 of four do not fit with one
 // CTA per SM (51 us a call).  A workspace of one row per CTA would be reproducible bit
@@ -22,8 +22,9 @@
 // multiply-adds of a warp) and by the latency of the eight products of a tile;
 // small batches are given one 16-sample tile per CTA to fill the SMs.  Measured
 // on B200, the whole call with its host read of the loss: 2048 samples (the
-// default batch) 42 us, 32,768 samples 103 us, against 13.1 and 13.7 ms for a
-// thread per sample with shared-memory atomics for every product.
+// default batch) 33.8 us, 32,768 samples 95 us, against 13.1 and 13.7 ms for a
+// thread per sample with shared-memory atomics for every product.  The rounding launch
+// writes the loss to pinned memory; a copy after it would make that 40.7 us.
 #pragma once
 #include <cuda_bf16.h>
 
@@ -248,10 +249,12 @@ __global__ void __launch_bounds__(mlpg::THREADS, 2)
   }
 }
 
-__global__ void mlp_grad_round_kernel(const double* sums, float* grad) {
+// grad = sums, rounded; the loss behind them to *loss (pinned host memory; may be null)
+__global__ void mlp_grad_round_kernel(const double* sums, float* grad, double* loss) {
   pdl_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < MLPDims::NPARAM) grad[i] = float(sums[i]);
+  else if (i == MLPDims::NPARAM && loss) *loss = sums[i];
 }
 
 }  // namespace sfem
