@@ -42,11 +42,10 @@ for p in (os.path.join(ROOT, "simplex-benchmarks_b200"), os.path.join(ROOT, "ora
 N_HEX, DEGREE, JITTER = 32, 3, 0.1
 METRIC = "vmult DoF/s (FP64 vs mixed); Poisson solve time to 1e-8 (MG vs learned)"
 WORKLOAD = "DG SIPG Poisson vmult, P3 on 32^3 x 6 Kuhn tets (196,608 cells, 3,932,160 DoFs), jitter 0.1h"
-# DRAM bytes (read + written) of one launch of the apply kernel on this
-# workload: dram__bytes_read.sum + dram__bytes_write.sum of an ncu capture
-# (profiles/dg_apply_kernel_p3_fp64_32cube.md)
+# DRAM bytes of the vmult's one launch on this workload: dram__bytes_read.sum +
+# dram__bytes_write.sum of an ncu capture of this kernel (blocks of 128 cells)
 VMULT_KERNEL = "dg_fused3_kernel<1,false,128,double,2>"
-VMULT_TRAFFIC_BYTES = 66.25e6  # captured with blocks of 64 cells
+VMULT_TRAFFIC_BYTES = 61.4e6
 
 
 def parse():
