@@ -81,15 +81,19 @@ typedef struct fem_op_params {
   int32_t n_components;    /* FEM_HELMHOLTZ: number of fields (reference: 3); others: 1 */
   int32_t penalty;         /* FEM_DG: enum fem_penalty */
   int32_t kernel_variant;  /* 0: tuned default; DG/Helmholtz: 1 one launch, thread per cell and
-                              component (vmult_phase: thread per cell x128), 2 thread per cell x64, 3 warp roles x32, 4 thread per cell
+                              component (vmult_phase: thread per cell x128; scalar P3 FP64
+                              with most neighbours outside a block: two launches), 2 thread
+                              per cell x64, 3 warp roles x32, 4 thread per cell
                               x64 with results in registers (scalar) and 8 CTAs per SM, 5 thread
                               per cell x64 with 5 CTAs per SM; CG: 1 thread per
                               cell (by patches of consecutive cells on larger meshes where 1
                               is the default), 2 thread per Kuhn hex (6 tets, one atomic per distinct
                               DoF), 3 CTA per 4x4x4 hexes (stores for interior DoFs: a thread
-                              per hex, or per tet for P3 FP64 and small P3 FP32 meshes); each
+                              per hex, or per tet for P3 FP64 and some P3 FP32 meshes); each
                               falls back to the next simpler form where the mesh lacks the
-                              pattern; default 3, and 1 on meshes with fewer than 148 blocks;
+                              pattern; default 3 on Kuhn boxes with enough hexes in full
+                              enough blocks (P3 FP64: 296 whole cubes), 2 on P1 boxes of
+                              50,000 hexes and more without, else 1;
                               4: FP32 CG on the TF32 tensor cores (tcgen05 kind::tf32, cell
                               operator as one [128 cells x K] x [K x 6K] product; ~1e-3
                               relative accuracy, for multigrid levels); CG 5, 6, 7: the cube

@@ -27,9 +27,12 @@
 // Measured on B200 against the thread-per-tet forms, back to back: P2 FP64 128^3
 // 343 -> 272 us, FP32 252 -> 155 us; P1 FP64 128^3 139 -> 101 us (the metric
 // alone is 92 us of HBM), FP32 74.5 -> 54 us; P3 FP32 64^3 100.6 -> 89.5 us; P2
-// FP64 on 37 x 41 x 35 hexes 18.7 -> 13.5 us.  What is left for P2 FP64 is
-// latency: 12 warps per SM of 168 registers, FP64 pipe 37 %, shared memory 53 %,
-// HBM 46 % busy.
+// FP64 on 37 x 41 x 35 hexes 18.7 -> 13.5 us.  What is left for P2 FP64 (128^3, by the
+// profiler) is latency: 12 warps per SM of 168 registers, 8.5 cycles an instruction;
+// FP64 pipe 35 %, L1 and shared memory 61 %, HBM 52 % busy (62 % of the bytes that the
+// kernel needs are the stored metric).  P3 FP32 64^3: 8 warps of 222 registers, 5.0
+// cycles, issue slots 40 %, L1 and shared memory 33 %.  Where the form is the default:
+// CGBlocks::pays.
 //
 // codes [n_blocks][NBP] DoF | interior << 30, -1: constrained or absent node
 // pos   [NBP]           lattice position of slot n (the same for every block;

@@ -15,9 +15,10 @@
 // B200, unstructured, 44 x 40 x 36 hexes' cells, us per vmult with the fill of dst, thread per
 // cell -> patches: P1 FP64 12.7 -> 8.4, FP32 12.8 -> 7.0; P2 FP64 22.7 -> 16.3, FP32 21.6 ->
 // 11.9; P3 FP64 48.5 -> 46, FP32 46.9 -> 33; three components P2 FP64 63.7 -> 49.7, FP32 61.2
-// -> 32.9.  P3 FP64 on 37 x 41 x 35 hexes 41 -> 35.  By the profiler (P2 FP64): shared
-// memory and L1 70 % (a third of the wavefronts are bank conflicts of the gather and
-// the sums), then the latency of the first loads; atomics down from 10 to 3.1 a cell.
+// -> 32.9.  P3 FP64 on 37 x 41 x 35 hexes 41 -> 35.  By the profiler (P2 FP64): the
+// latency of the first loads (7 of 15 cycles an instruction at 12 to 14 warps per SM), L1
+// 62 % (a third of the wavefronts are bank conflicts of the gather and the sums);
+// atomics down from 10 to 3.1 a cell.
 #pragma once
 #include <cstdint>
 

@@ -27,9 +27,9 @@
 // nothing is waited for after the one staging (loading it face by face instead:
 // P2 FP64, three components 117 us, neighbours from global memory too 115 us,
 // staged 80 us).  The faces come first, then the cell term, which keeps the live
-// values to about 50.  What is left for P2 FP64, three components: shared-memory
-// wavefronts 64 %, issue slots 46 %, FP64 pipe 40 % busy; in FP32 the issue slots
-// (72 %).  Persistent CTAs that copy the next block during the arithmetic were not
+// values to about 50.  What is left by the profiler (cold caches) for P2 FP64, three
+// components: shared-memory wavefronts 69 %, issue slots 49 %, FP64 pipe 42 % busy; for
+// scalar P2 FP32 the issue slots (65 %).  Persistent CTAs that copy the next block during the arithmetic were not
 // faster (105 us: the second stage costs resident warps).
 #pragma once
 #include <cstdint>

@@ -16,11 +16,11 @@
 // a cell and component, written once and read twice) and the waits for
 // neighbours in other CTAs, one per face.  B200, 45 x 38 x 31 hexes, us per vmult,
 // two launches -> one: DG FP64 97 -> 66, FP32 55 -> 38; Helmholtz, 3 components,
-// FP64 526 -> 231, FP32 252 -> 122.  32^3 by the profiler: 19.8 M warp
-// instructions, FP64 pipe 32 %, issue slots 38 %, shared memory 42 %, 224
-// registers and 52 KB per 64 cells, so 8 warps an SM: bound by latency, the copies'
-// first (30 % of the cycles before the outer rows' indices were requested all at
-// once, which took FP64 from 77 to 66 us).
+// FP64 526 -> 231, FP32 252 -> 122.  FP64 32^3 by the profiler: 18.8 M warp
+// instructions, FP64 pipe 36 %, issue slots 40 %, shared memory 47 %; 224 registers and
+// 93 KB per CTA of 128 cells leave two of them an SM, 8 warps: bound by latency, 4.6
+// cycles an instruction (the copies took 30 % of the cycles before the outer rows'
+// indices were requested all at once, which took FP64 from 77 to 66 us).
 #pragma once
 #include <cstdint>
 
