@@ -488,7 +488,7 @@ class CGOperator final : public Operator {
 
   // the tables that only variant v's form reads
   void make_tables(int v) {
-    if (v == 0) v = default_variant();
+    if (v == 0) v = default_form;
     if (v == 3 && use_blocks()) blocks.make_metric(d_geo);
     else if (v == 2 || ((v == 3 || (v >= 5 && v <= 7)) && !cube_NB)) make_hex_tables();
   }
@@ -548,7 +548,8 @@ class CGOperator final : public Operator {
     find_hex_pattern(mesh, dofs);
     build_cube_tables(dofs);
     blocks.build(mesh, cfg.degree, dofs.cell_dofs, dofs.constrained);
-    if (default_variant() == 1) patches.build(cfg.degree, K, n_cells, dofs.cell_dofs, dofs.constrained);
+    default_form = default_variant();
+    if (default_form == 1) patches.build(cfg.degree, K, n_cells, dofs.cell_dofs, dofs.constrained);
     if (cfg.weak_bc) build_weak_boundary(mesh);
     d_status.alloc(1);
     SFEM_CUDA(cudaMemset(d_status.p, 0, sizeof(int)));
@@ -682,6 +683,7 @@ class CGOperator final : public Operator {
   // 37^3 7.1 / 7.5, 32^3 6.6 / 5.9); else 1, which is cg_patch_kernel if the mesh has
   // enough patches (CGPatches), or a thread per cell.  P3 FP64 without whole cubes: 37 x
   // 41 x 35 hexes 41.5 us by cells, per hex 49.5 us.
+  int default_form = 1;  // default_variant(), once at set-up
   int default_variant() const {
     if (blocks.pays(cfg.degree)) return 3;
     if (cfg.degree == 3 && cube_NB && n_blocks >= 2 * 148) return 3;
@@ -710,7 +712,7 @@ class CGOperator final : public Operator {
       launch_tc_cell(x, d, s);
       return;
     }
-    if (v == 0) v = default_variant();
+    if (v == 0) v = default_form;
     // variant 3: the block form where it is the faster one, else the cube kernel;
     // cube reduce schedule: variants 5, 6, 7 pick one; variant 3 takes the one
     // measured fastest on B200 (FP64 P1 and P2: bank-scheduled with uniform steps;
@@ -777,7 +779,7 @@ class CGOperator final : public Operator {
   bool block_form() const override { return use_blocks() && blocks.n_blocks >= 148; }
   // default variant; 3 is the block form, cubes, hexes; 1 is the patch form
   std::string forms() const override {
-    return std::to_string(default_variant()) + (use_blocks() ? "b" : "") + (cube_NB ? "c" : "") + (hex_H ? "h" : "") +
+    return std::to_string(default_form) + (use_blocks() ? "b" : "") + (cube_NB ? "c" : "") + (hex_H ? "h" : "") +
            (patches.n_patches ? "p" : "");
   }
   const BlockView* block_view() const override { return blocks.view.n_blocks ? &blocks.view : nullptr; }
@@ -802,7 +804,7 @@ class CGOperator final : public Operator {
   // index and metric tables that the current form reads
   size_t table_bytes() const {
     const size_t metric = d_geo.n * sizeof(T);
-    int v = cfg.kernel_variant == 0 ? default_variant() : cfg.kernel_variant;
+    const int v = cfg.kernel_variant == 0 ? default_form : cfg.kernel_variant;
     if (v == 3 && use_blocks()) return blocks.table_bytes();
     if ((v == 3 || v >= 5) && cube_NB) return metric + d_bdof.n * sizeof(int32_t);
     if (v == 2 || v == 3 || (v >= 5 && v <= 7))
@@ -829,6 +831,7 @@ class CGVectorOperator final : public Operator {
   std::vector<int32_t> node_dofs;  // [n_cells][K]
   CGBlocks<T, NC> blocks;          // 4 x 4 x 4-hex blocks (Kuhn boxes)
   CGPatches<T, NC> patches;        // patches of cells elsewhere
+  bool blocks_pay = false;         // the block form is the default
 
   CGVectorOperator(const Mesh& mesh, const OpConfig& c) {
     cfg = c;
@@ -870,13 +873,14 @@ class CGVectorOperator final : public Operator {
     d_geo.upload(geo);
     d_constrained.upload(cl);
     blocks.build(mesh, cfg.degree, dofs.cell_dofs, dofs.constrained);
+    blocks_pay = blocks.pays(cfg.degree);
     make_tables(cfg.kernel_variant);
     // P3 FP64 keeps the thread per cell: 44 x 40 x 36 hexes 130 us, by patches 137 to 160
-    if (!blocks.pays(cfg.degree) && (cfg.degree <= 2 || sizeof(T) == 4))
+    if (!blocks_pay && (cfg.degree <= 2 || sizeof(T) == 4))
       patches.build(cfg.degree, K, n_cells, dofs.cell_dofs, dofs.constrained);
   }
   void make_tables(int v) {
-    if (v == 3 || (v == 0 && blocks.pays(cfg.degree))) blocks.make_metric(d_geo);
+    if (v == 3 || (v == 0 && blocks_pay)) blocks.make_metric(d_geo);
   }
   std::mutex tables_mutex;
   void set_variant(int v) override {
@@ -889,7 +893,7 @@ class CGVectorOperator final : public Operator {
   }
   bool block_form() const override { return blocks.n_blocks >= 148; }
   std::string forms() const override {
-    return std::string(blocks.pays(cfg.degree) ? "3" : "1") + (blocks.n_blocks ? "b" : "") +
+    return std::string(blocks_pay ? "3" : "1") + (blocks.n_blocks ? "b" : "") +
            (patches.n_patches ? "p" : "");
   }
 
@@ -906,7 +910,7 @@ class CGVectorOperator final : public Operator {
       return;
     }
     const int v = cfg.kernel_variant;
-    if (blocks.n_blocks && (v == 3 || (v == 0 && blocks.pays(cfg.degree)))) {
+    if (blocks.n_blocks && (v == 3 || (v == 0 && blocks_pay))) {
       blocks.launch(cfg.degree, x, d, d_constrained.n, d_constrained.p, s);
       return;
     }
@@ -951,7 +955,7 @@ class CGVectorOperator final : public Operator {
     const int p = cfg.degree, kq = kq_of(p);
     flops = NC * 2.0 * (2 * nnz_grad_rt(p) + 9 * kq + 3 * kq * kq) * double(n_cells);
     const int v = cfg.kernel_variant;
-    const bool by_blocks = blocks.n_blocks && (v == 3 || (v == 0 && blocks.pays(p)));
+    const bool by_blocks = blocks.n_blocks && (v == 3 || (v == 0 && blocks_pay));
     const size_t tables = by_blocks ? blocks.table_bytes()
                                     : d_geo.n * sizeof(T) + (patches.n_patches ? patches.table_bytes()
                                                                                : d_dofs.n * sizeof(int32_t));
